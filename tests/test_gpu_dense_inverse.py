@@ -1,0 +1,29 @@
+"""The coarsest level's Cholesky factor and inverse, kernel by kernel, at sizes
+around their 32-column blocks, 64-wide tiles and 128-column steps: A A^-1 = I
+on well-conditioned matrices (condition below 4; the residual of an explicit
+inverse through its Cholesky factor is of the order of n eps cond, 4 n eps is
+asked for), exact symmetry, no pivot flagged."""
+import shutil
+import subprocess
+from pathlib import Path
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+ROOT = Path(__file__).resolve().parents[1]
+SIZES = [1, 31, 32, 33, 63, 64, 65, 127, 128, 129, 160, 255, 257, 300, 449]
+
+
+def test_factor_and_inverse(tmp_path):
+    nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
+    exe = tmp_path / "dense_harness"
+    subprocess.run([nvcc, "-gencode", "arch=compute_100a,code=sm_100a", "-O2", "-std=c++17", "--expt-relaxed-constexpr",
+                    "-I", str(ROOT / "include"), "-I", str(ROOT / "top_gpu_on_matlab_b200" / "csrc"), "-o", str(exe),
+                    str(ROOT / "tests" / "dense_harness.cu")], check=True)
+    out = subprocess.run([str(exe)] + [str(n) for n in SIZES], check=True, capture_output=True, text=True, timeout=120).stdout
+    rows = [line.split() for line in out.splitlines()]
+    assert [int(r[0]) for r in rows] == SIZES
+    for n, res, asym, status in rows:
+        assert float(res) <= max(4, 4 * int(n)) * np.finfo(float).eps, (n, res)
+        assert float(asym) == 0.0 and int(status) == 0, (n, asym, status)

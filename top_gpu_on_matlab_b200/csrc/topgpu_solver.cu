@@ -1223,6 +1223,9 @@ extern "C" int top_solver_destroy(top_solver *s)
     if (s->capStream) cudaStreamDestroy(s->capStream);
     if (s->capIn) cudaEventDestroy(s->capIn);
     if (s->capOut) cudaEventDestroy(s->capOut);
+    if (s->auxStream) cudaStreamDestroy(s->auxStream);
+    if (s->auxGo) cudaEventDestroy(s->auxGo);
+    if (s->auxDone) cudaEventDestroy(s->auxDone);
     for (auto &k : s->l0k) if (k.mask) cudaFree(k.mask);
     if (s->l0kFallback.mask) cudaFree(s->l0kFallback.mask);
     for (void *p : s->allocs) cudaFree(p);
@@ -1346,15 +1349,17 @@ extern "C" int top_solver_set_density(top_solver *s, const double *x, int where)
 // s->Ainv (which also serves as the product scratch of the inversion);
 // a non-positive pivot sets s->zeroDone[1]
 namespace {
+// C = A B^T on the tiled tensor-core product: (ta, tb) as dgemm_tile_kernel's;
+// lower / mirror / kFromTile likewise
 void dgemm(cudaStream_t st, bool ta, bool tb, double *C, int64_t ldc, const double *A, int64_t lda, const double *B, int64_t ldb,
-           int64_t M, int64_t N, int64_t K, double alpha, double beta, bool lower, bool kFromTile)
+           int64_t M, int64_t N, int64_t K, bool lower, bool mirror, bool kFromTile)
 {
     if (M <= 0 || N <= 0) return;
-    const dim3 g((unsigned)((M + 63) / 64), (unsigned)((N + 63) / 64));
-    const int lo = lower ? 1 : 0, kt = kFromTile ? 1 : 0;
-    if (!ta && !tb) dgemm_tile_kernel<false, false><<<g, 256, 0, st>>>(C, ldc, A, lda, B, ldb, (int)M, (int)N, (int)K, alpha, beta, lo, kt);
-    else if (!ta && tb) dgemm_tile_kernel<false, true><<<g, 256, 0, st>>>(C, ldc, A, lda, B, ldb, (int)M, (int)N, (int)K, alpha, beta, lo, kt);
-    else dgemm_tile_kernel<true, true><<<g, 256, 0, st>>>(C, ldc, A, lda, B, ldb, (int)M, (int)N, (int)K, alpha, beta, lo, kt);
+    const dim3 g((unsigned)((M + kTileB - 1) / kTileB), (unsigned)((N + kTileB - 1) / kTileB));
+    const int lo = lower ? 1 : 0, mi = mirror ? 1 : 0, kt = kFromTile ? 1 : 0;
+    if (!ta && !tb) dgemm_tile_kernel<false, false><<<g, kTileThreads, 0, st>>>(C, ldc, A, lda, B, ldb, (int)M, (int)N, (int)K, lo, mi, kt);
+    else if (!ta && tb) dgemm_tile_kernel<false, true><<<g, kTileThreads, 0, st>>>(C, ldc, A, lda, B, ldb, (int)M, (int)N, (int)K, lo, mi, kt);
+    else dgemm_tile_kernel<true, true><<<g, kTileThreads, 0, st>>>(C, ldc, A, lda, B, ldb, (int)M, (int)N, (int)K, lo, mi, kt);
 }
 }  // namespace
 
@@ -1436,8 +1441,8 @@ int build_tail(top_solver *s, cudaStream_t st)
         coarsest_assemble_kernel<<<(unsigned)((n + 7) / 8), 256, 0, st>>>(lv.KsC, lv.nodeGrid, s->tailEleCompact[k], s->tailNodeCompact[k], lv.g, lv.Nn, K);
         tail_jacobi_kernel<<<nb256(n), 256, 0, st>>>(s->tailJ, lv.invD64, lv.nodeGrid, lv.Nn, lv.g.cs, s->p.omega);
         tail_q_kernel<<<nb256(n * m), 256, 0, st>>>(s->tailQ, s->tailPt[k], K, s->tailJ, s->tailNbr[k], n, m);
-        dgemm(st, false, true, s->tailT, n, s->tailQ, n, Mnext, m, n, m, m, 1.0, 0.0, false, false);   // T = Q M'
-        dgemm(st, false, false, M, n, s->tailT, n, s->tailQ, n, n, n, m, 1.0, 0.0, true, false);      // T Q^T, lower
+        dgemm(st, false, true, s->tailT, n, s->tailQ, n, Mnext, m, n, m, m, false, false, false);   // T = Q M'
+        dgemm(st, false, false, M, n, s->tailT, n, s->tailQ, n, n, n, m, true, false, false);      // T Q^T, lower
         tail_m_kernel<<<nb256(n * n), 256, 0, st>>>(M, K, s->tailJ, n);
         s->launches += 6;
         Mnext = M;
@@ -1457,18 +1462,36 @@ int coarsest_inverse(top_solver *s, cudaStream_t st)
 {
     const int64_t n = s->nC, nblk = (n + kDb - 1) / kDb;
     double *A = s->Ac;
-    for (int64_t b = 0; b < nblk; ++b) {
-        const int64_t k0 = b * kDb;
-        const int kb = (int)std::min<int64_t>(kDb, n - k0);
-        double *D = s->Dc + b * kDb * kDb;
-        chol_block_kernel<<<1, 32, 0, st>>>(A, n, k0, kb, D, s->zeroDone + 1);
+    static const bool attr = cudaFuncSetAttribute(chol_diag_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDiagSmem) == cudaSuccess &&
+                             cudaFuncSetAttribute(chol_panel_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPanelSmem) == cudaSuccess;
+    if (!attr) { set_error("top_solver_assemble: shared memory of the coarsest factorisation"); return TOP_ERR_CUDA; }
+    // Each step's trailing update is split: the next step's 128 columns first, on
+    // the caller's stream, then the rest on a second stream, beside the next
+    // diagonal block (one CTA, 53 us) and panel, which touch other columns.
+    if (n > 2 * kPb && !s->auxStream) {
+        CK(cudaStreamCreateWithFlags(&s->auxStream, cudaStreamNonBlocking));
+        CK(cudaEventCreateWithFlags(&s->auxGo, cudaEventDisableTiming));
+        CK(cudaEventCreateWithFlags(&s->auxDone, cudaEventDisableTiming));
+    }
+    constexpr int kNext = kPb / kTileB;                // tile columns of the next step
+    bool restRuns = false;
+    for (int64_t k0 = 0; k0 < n; k0 += kPb) {
+        chol_diag_kernel<<<1, kDiagThreads, kDiagSmem, st>>>(A, n, k0, s->Dc, s->zeroDone + 1);
         TOPGPU_COUNT_LAUNCH();
-        const int64_t rest = n - k0 - kb;
-        if (rest > 0) {
-            double *L21 = A + (k0 + kb) + n * k0;
-            dgemm(st, false, false, L21, n, L21, n, D, kDb, rest, kb, kb, 1.0, 0.0, false, false);       // A21 L11^-T
-            dgemm(st, false, false, A + (k0 + kb) * (1 + n), n, L21, n, L21, n, rest, rest, kb, -1.0, 1.0, true, false);
-            s->launches += 2;
+        const int64_t rest = n - k0 - kPb;
+        if (rest <= 0) break;
+        const int nt = (int)((rest + kTileB - 1) / kTileB);
+        chol_panel_kernel<<<(unsigned)nt, kPanelThreads, kPanelSmem, st>>>(A, n, k0, s->Dc);
+        if (nt > kNext) CK(cudaEventRecord(s->auxGo, st));                 // the panel is complete
+        if (restRuns) CK(cudaStreamWaitEvent(st, s->auxDone, 0));          // the previous step's updates of these columns
+        chol_trail_kernel<<<dim3((unsigned)nt, (unsigned)std::min(nt, kNext)), kTileThreads, 0, st>>>(A, n, k0, 0);
+        s->launches += 2;
+        restRuns = nt > kNext;
+        if (restRuns) {
+            CK(cudaStreamWaitEvent(s->auxStream, s->auxGo, 0));
+            chol_trail_kernel<<<dim3((unsigned)nt, (unsigned)(nt - kNext)), kTileThreads, 0, s->auxStream>>>(A, n, k0, kNext);
+            TOPGPU_COUNT_LAUNCH();
+            CK(cudaEventRecord(s->auxDone, s->auxStream));
         }
     }
     CK(cudaMemsetAsync(s->Wc, 0, sizeof(double) * n * n, st));
@@ -1477,11 +1500,11 @@ int coarsest_inverse(top_solver *s, cudaStream_t st)
     for (int64_t hs = kDb; hs < n; hs *= 2) {          // bottom-up levels of the block inversion
         const int64_t nodes = (n + 2 * hs - 1) / (2 * hs), tiles = (hs + 63) / 64;
         for (int step = 0; step < 2; ++step) {
-            inv_level_kernel<<<dim3((unsigned)tiles, (unsigned)tiles, (unsigned)nodes), 256, 0, st>>>(A, s->Wc, s->Ainv, n, (int)hs, step);
+            inv_level_kernel<<<dim3((unsigned)tiles, (unsigned)tiles, (unsigned)nodes), kTileThreads, 0, st>>>(A, s->Wc, s->Ainv, n, (int)hs, step);
             TOPGPU_COUNT_LAUNCH();
         }
     }
-    dgemm(st, true, true, s->Ainv, n, s->Wc, n, s->Wc, n, n, n, n, 1.0, 0.0, false, true);         // W^T W
+    dgemm(st, true, true, s->Ainv, n, s->Wc, n, s->Wc, n, n, n, n, false, true, true);         // W^T W
     TOPGPU_COUNT_LAUNCH();
     return TOP_OK;
 }
