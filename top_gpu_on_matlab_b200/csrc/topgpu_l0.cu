@@ -152,10 +152,8 @@ void l0_op(top_solver *s, const In &in, const Out &out, Reduce red, const int *d
     const top_solver::L0Kernel &k = s->l0k[prec_slot<T>()];
     const unsigned K = (unsigned)nv;  // right-hand sides (grid y or z)
     if (s->super) {                   // per-element matrices (K_mat), packed on the grid
-        const T *Kp;
-        if constexpr (sizeof(T) == 8) Kp = lv.KsP64; else Kp = lv.KsP32;
-        dim3 gr = coarse_tile_grid(lv.g); gr.z = K;
-        launch_k(s, coarse_tile_kernel<T, In, Out>, gr, dim3(kCoarseTileX, 8), 0, s->st, in, out, Kp, lv.g, red, done);
+        packed_op<T>(s, lv, in, out, red, done, nv);
+        return;
     } else if (k.kind == 1) {
 #define TOPGPU_LAUNCH_SHAPE(A, B)                                                                             \
         if (k.ty == A && k.tx == B)                                                                           \

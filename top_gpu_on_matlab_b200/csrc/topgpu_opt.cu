@@ -56,7 +56,8 @@ struct SFilterState {
     bool ready = false;
     double rMin = 0;
     int R = 0, fy = 0, fx = 0, fz = 0;
-    double *h = nullptr, *Hs = nullptr, *g = nullptr, *t = nullptr;
+    double *h = nullptr, *g = nullptr;   // taps and the operand with its margin, sized by R (freed with the state)
+    double *Hs = nullptr;                // element-major
 };
 
 struct OptState {
@@ -323,58 +324,96 @@ __global__ void fpcg_start_kernel(PcgState *st, double tol, int maxIT)
 }
 
 // ---- super-element density filter ---------------------------------------------
-// sub-voxel (q, e) of the element-major [64 x Ne] layout <-> fine-grid voxel
-// (y fastest); q = ly + 4 (lx + 4 lz) (gen_index_mapping, TOP_GPU.m:2673-2697)
-__device__ __forceinline__ int64_t sub_to_fine(int64_t i, int ny, int nx, int fy, int fx)
+// sub-voxel i = q + 64 e of the element-major [64 x Ne] layout -> its fine-grid
+// coordinates; q = ly + 4 (lx + 4 lz) (gen_index_mapping, TOP_GPU.m:2673-2697)
+__device__ __forceinline__ void sub_to_fine(int64_t i, int ny, int nx, int &y, int &x, int &z)
 {
     const int64_t e = i / 64; const int q = (int)(i % 64);
     const int ey = (int)(e % ny), ex = (int)((e / ny) % nx), ez = (int)(e / ((int64_t)ny * nx));
-    const int y = 4 * ey + (q & 3), x = 4 * ex + ((q >> 2) & 3), z = 4 * ez + (q >> 4);
-    return y + (int64_t)fy * (x + (int64_t)fx * z);
+    y = 4 * ey + (q & 3); x = 4 * ex + ((q >> 2) & 3); z = 4 * ez + (q >> 4);
 }
-// mode 0: g = in ./ Hs (sensitivities), mode 1: g = in (densities)
+// the correlation's operand: the fine grid with x fastest inside a margin of
+// R zeros (kSfRows - 1 more past the last y, for the last thread's rows)
+constexpr int kSfRows = 8;
+struct SfGeom {
+    int fy, fx, fz, R;
+    __host__ __device__ int px() const { return fx + 2 * R; }
+    __host__ __device__ int py() const { return fy + 2 * R + kSfRows - 1; }
+    __host__ __device__ int64_t size() const { return (int64_t)px() * py() * (fz + 2 * R); }
+    // first tap of output (y, x, z): operand entry (y - R, x - R, z - R)
+    __host__ __device__ int64_t at(int y, int x, int z) const { return x + (int64_t)px() * (y + (int64_t)py() * z); }
+};
+// mode 0: g = in ./ Hs (sensitivities), mode 1: g = in (densities); Hs in the
+// element-major order of in (mode 0 with Hs null: ones)
 __global__ void sfilt_gather_kernel(const double *__restrict__ in, const double *__restrict__ Hs, int mode, int ny, int nx,
-                                    int fy, int fx, int64_t n, double *__restrict__ g)
+                                    SfGeom s, int64_t n, double *__restrict__ g)
 {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    const int64_t f = sub_to_fine(i, ny, nx, fy, fx);
-    g[f] = mode == 0 ? in[i] / Hs[f] : in[i];
+    int y, x, z;
+    sub_to_fine(i, ny, nx, y, x, z);
+    g[s.at(y + s.R, x + s.R, z + s.R)] = mode == 0 ? in[i] / Hs[i] : in[i];
 }
-__global__ void sfilt_scatter_kernel(const double *__restrict__ t, const double *__restrict__ Hs, int mode, int ny, int nx,
-                                     int fy, int fx, int64_t n, double *__restrict__ out)
+// t = imfilter(g, h): correlation, zero outside (the kernel is symmetric), and
+// out = t (mode 0) or t ./ Hs (mode 1), element-major.  FP64-issue bound: (2R+1)^3
+// multiply-adds an output.  A thread forms YB outputs consecutive in y with its
+// lanes along x (coalesced operand rows); for each (dz, dx) it slides over the
+// 2R + YB operand rows in groups of four taps, so a group costs 4 operand and
+// 4 tap loads for 4 YB multiply-adds; the loads' L1 wavefronts bound it now.  On
+// the 40x240x40 fine grid at R = 6: 633 us (one output a thread, two loads a
+// multiply-add behind bounds checks) -> 219 us, the whole filter 638 -> 240 us.
+// The multiply-adds run in the order dz, dx, dy ascending; taps outside the
+// grid read the zero margin.
+template <int YB>
+__global__ void __launch_bounds__(128)
+sfilt_conv_kernel(const double *__restrict__ g, const double *__restrict__ h, SfGeom s, const double *__restrict__ Hs, int mode,
+                  int ny, int nx, double *__restrict__ out)
 {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const int64_t f = sub_to_fine(i, ny, nx, fy, fx);
-    out[i] = mode == 1 ? t[f] / Hs[f] : t[f];
-}
-// t = imfilter(g, h): correlation, zero outside (the kernel is symmetric)
-__global__ void sfilt_conv_kernel(const double *__restrict__ g, const double *__restrict__ h, int R, int fy, int fx, int fz,
-                                  double *__restrict__ t)
-{
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const int64_t n = (int64_t)fy * fx * fz;
-    if (i >= n) return;
-    const int y = (int)(i % fy), x = (int)((i / fy) % fx), z = (int)(i / ((int64_t)fy * fx));
-    const int w = 2 * R + 1;
-    double s = 0;
-    for (int dz = -R; dz <= R; ++dz) {
-        const int zz = z + dz;
-        if (zz < 0 || zz >= fz) continue;
-        for (int dx = -R; dx <= R; ++dx) {
-            const int xx = x + dx;
-            if (xx < 0 || xx >= fx) continue;
-            const double *gr = g + (int64_t)fy * (xx + (int64_t)fx * zz);
-            const double *hr = h + w * ((dx + R) + w * (dz + R)) + R;
-            for (int dy = -R; dy <= R; ++dy) {
-                const int yy = y + dy;
-                if (yy < 0 || yy >= fy) continue;
-                s = fma(gr[yy], hr[dy], s);
+    const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int ng = (s.fy + YB - 1) / YB;
+    if (k >= (int64_t)s.fx * ng * s.fz) return;
+    const int x = (int)(k % s.fx), y0 = (int)((k / s.fx) % ng) * YB, z = (int)(k / ((int64_t)s.fx * ng));
+    const int w = 2 * s.R + 1, px = s.px();
+    double acc[YB];
+#pragma unroll
+    for (int u = 0; u < YB; ++u) acc[u] = 0.0;
+    for (int dz = 0; dz < w; ++dz)
+        for (int dx = 0; dx < w; ++dx) {
+            const double *gr = g + s.at(y0, x + dx, z + dz);
+            const double *hr = h + w * (dx + w * dz);
+            double win[YB + 3];
+#pragma unroll
+            for (int u = 0; u < YB - 1; ++u) win[u] = gr[(int64_t)px * u];
+            int dy = 0;
+            for (; dy + 4 <= w; dy += 4) {
+#pragma unroll
+                for (int u = 0; u < 4; ++u) win[YB - 1 + u] = gr[(int64_t)px * (dy + YB - 1 + u)];
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const double hv = hr[dy + q];
+#pragma unroll
+                    for (int u = 0; u < YB; ++u) acc[u] = fma(win[u + q], hv, acc[u]);
+                }
+#pragma unroll
+                for (int u = 0; u < YB - 1; ++u) win[u] = win[u + 4];
+            }
+            for (; dy < w; ++dy) {
+                win[YB - 1] = gr[(int64_t)px * (dy + YB - 1)];
+                const double hv = hr[dy];
+#pragma unroll
+                for (int u = 0; u < YB; ++u) acc[u] = fma(win[u], hv, acc[u]);
+#pragma unroll
+                for (int u = 0; u < YB - 1; ++u) win[u] = win[u + 1];
             }
         }
+#pragma unroll
+    for (int u = 0; u < YB; ++u) {
+        const int y = y0 + u;
+        if (y >= s.fy) break;
+        const int64_t e = (y >> 2) + (int64_t)ny * ((x >> 2) + (int64_t)nx * (z >> 2));
+        const int64_t i = 64 * e + (y & 3) + 4 * ((x & 3) + 4 * (z & 3));
+        out[i] = mode == 1 ? acc[u] / Hs[i] : acc[u];
     }
-    t[i] = s;
 }
 
 // ---- sensitivities ----------------------------------------------------------
@@ -617,6 +656,7 @@ void topgpu::free_opt_state(top_solver *s)
     if (s->filterState && filt(s).chunk) cudaGraphExecDestroy(filt(s).chunk);
     delete reinterpret_cast<FilterState *>(s->filterState);
     if (s->optState && opt(s).sf.h) cudaFree(opt(s).sf.h);
+    if (s->optState && opt(s).sf.g) cudaFree(opt(s).sf.g);
     delete reinterpret_cast<OptState *>(s->optState);
     delete reinterpret_cast<AdjState *>(s->adjState);
     s->filterState = s->optState = s->adjState = nullptr;
@@ -740,6 +780,19 @@ extern "C" int top_solver_filter(top_solver *s, const double *src, double *tar, 
 }
 
 // ---- super-element density filter (host side) --------------------------------
+// out = imfilter(f.g, h), ./ Hs in mode 1.  Eight outputs a thread where that
+// still gives every scheduler two warps (the 40x240x40 fine grid and up), else four.
+static void sfilt_conv(top_solver *s, const double *Hs, int mode, double *out)
+{
+    SFilterState &f = opt(s).sf;
+    const SfGeom sg{f.fy, f.fx, f.fz, f.R};
+    const int64_t cols = (int64_t)f.fx * f.fz, n8 = cols * ((f.fy + 7) / 8), n4 = cols * ((f.fy + 3) / 4);
+    if (n8 >= (int64_t)s->numSMs * 4 * 2 * 32)
+        sfilt_conv_kernel<8><<<(unsigned)((n8 + 127) / 128), 128, 0, s->st>>>(f.g, f.h, sg, Hs, mode, s->nely, s->nelx, out);
+    else
+        sfilt_conv_kernel<4><<<(unsigned)((n4 + 127) / 128), 128, 0, s->st>>>(f.g, f.h, sg, Hs, mode, s->nely, s->nelx, out);
+    TOPGPU_COUNT_LAUNCH();
+}
 static int sfilter_setup(top_solver *s, double rMin)
 {
     OptState &o = opt(s);
@@ -754,8 +807,8 @@ static int sfilter_setup(top_solver *s, double rMin)
     f.fy = 4 * s->nely; f.fx = 4 * s->nelx; f.fz = 4 * s->nelz;
     const int64_t N = (int64_t)f.fy * f.fx * f.fz;
     if (!f.Hs) {
-        f.Hs = s->dalloc<double>(N); f.g = s->dalloc<double>(N); f.t = s->dalloc<double>(N);
-        if (!f.Hs || !f.g || !f.t) { set_error("super-element filter: out of device memory"); return TOP_ERR_NOMEM; }
+        f.Hs = s->dalloc<double>(N);
+        if (!f.Hs) { set_error("super-element filter: out of device memory"); return TOP_ERR_NOMEM; }
     }
     std::vector<double> h((size_t)w * w * w);
     for (int dz = -f.R; dz <= f.R; ++dz)
@@ -764,13 +817,21 @@ static int sfilter_setup(top_solver *s, double rMin)
                 const double v = r - std::sqrt(double(dx * dx + dy * dy + dz * dz));
                 h[(dy + f.R) + w * ((dx + f.R) + w * (dz + f.R))] = v > 0 ? v : 0.0;
             }
+    f.ready = false;
     if (f.h) cudaFree(f.h);
+    if (f.g) cudaFree(f.g);
+    f.h = f.g = nullptr;
+    const SfGeom sg{f.fy, f.fx, f.fz, f.R};
     if (cudaMalloc(&f.h, sizeof(double) * h.size()) != cudaSuccess) { f.h = nullptr; return TOP_ERR_NOMEM; }
+    if (cudaMalloc(&f.g, sizeof(double) * sg.size()) != cudaSuccess) { f.g = nullptr; return TOP_ERR_NOMEM; }
     CK(cudaMemcpyAsync(f.h, h.data(), sizeof(double) * h.size(), cudaMemcpyHostToDevice, s->st));
-    fill_kernel<<<vb(N), 256, 0, s->st>>>(f.g, 1.0, N);
+    CK(cudaMemsetAsync(f.g, 0, sizeof(double) * sg.size(), s->st));
+    // Hs = imfilter(ones, h): the operand filled with ones (Hs holds them first)
+    fill_kernel<<<vb(N), 256, 0, s->st>>>(f.Hs, 1.0, N);
     TOPGPU_COUNT_LAUNCH();
-    sfilt_conv_kernel<<<(unsigned)((N + 255) / 256), 256, 0, s->st>>>(f.g, f.h, f.R, f.fy, f.fx, f.fz, f.Hs);
+    sfilt_gather_kernel<<<(unsigned)((N + 255) / 256), 256, 0, s->st>>>(f.Hs, nullptr, 1, s->nely, s->nelx, sg, N, f.g);
     TOPGPU_COUNT_LAUNCH();
+    sfilt_conv(s, nullptr, 0, f.Hs);
     CK(cudaStreamSynchronize(s->st));      // h (host vector) is consumed
     f.rMin = rMin;
     f.ready = true;
@@ -780,13 +841,11 @@ static int sfilter_setup(top_solver *s, double rMin)
 static int sfilter_apply(top_solver *s, const double *in, double *out, int mode)
 {
     SFilterState &f = opt(s).sf;
-    const int64_t n = 64 * s->L[0].Ne, N = (int64_t)f.fy * f.fx * f.fz;
-    sfilt_gather_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s->st>>>(in, f.Hs, mode, s->nely, s->nelx, f.fy, f.fx, n, f.g);
+    const int64_t n = 64 * s->L[0].Ne;
+    const SfGeom sg{f.fy, f.fx, f.fz, f.R};
+    sfilt_gather_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s->st>>>(in, f.Hs, mode, s->nely, s->nelx, sg, n, f.g);
     TOPGPU_COUNT_LAUNCH();
-    sfilt_conv_kernel<<<(unsigned)((N + 255) / 256), 256, 0, s->st>>>(f.g, f.h, f.R, f.fy, f.fx, f.fz, f.t);
-    TOPGPU_COUNT_LAUNCH();
-    sfilt_scatter_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s->st>>>(f.t, f.Hs, mode, s->nely, s->nelx, f.fy, f.fx, n, out);
-    TOPGPU_COUNT_LAUNCH();
+    sfilt_conv(s, f.Hs, mode, out);
     CK(cudaGetLastError());
     return TOP_OK;
 }

@@ -4,6 +4,7 @@
 #pragma once
 #include <cuda_runtime.h>
 #include <nvtx3/nvToolsExt.h>
+#include <algorithm>
 #include <cstdlib>
 #include <vector>
 #include <utility>
@@ -191,6 +192,61 @@ inline void launch_k(const top_solver *s, void (*kernel)(KArgs...), dim3 grid, d
 
 // every kernel launch of the solver is counted on the solver it serves
 #define TOPGPU_COUNT_LAUNCH() (++s->launches)
+
+namespace topgpu {
+// ---- products with packed element matrices: every coarse level, and level 0
+// in super-element mode ----
+template <typename T> inline const T *ks_packed(const DevLevel &l);
+template <> inline const double *ks_packed<double>(const DevLevel &l) { return l.KsP64; }
+template <> inline const float *ks_packed<float>(const DevLevel &l) { return l.KsP32; }
+template <typename T> inline T *wbuf(DevLevel &l);
+template <> inline double *wbuf<double>(DevLevel &l) { return l.W64; }
+template <> inline float *wbuf<float>(DevLevel &l) { return l.W32; }
+// resident CTAs per SM of the two-pass product's first pass (its dynamic
+// shared memory allowance set once; 0 when that fails)
+template <typename T, class In>
+inline int coarse_elem_occ()
+{
+    static const int occ = [] {
+        int n = 0;
+        if (cudaFuncSetAttribute(coarse_elem_kernel<T, In>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CoarseElem<T>::kSmem) != cudaSuccess ||
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, coarse_elem_kernel<T, In>, kElemThreads, CoarseElem<T>::kSmem) != cudaSuccess) {
+            (void)cudaGetLastError();
+            n = 0;
+        }
+        return n;
+    }();
+    return occ;
+}
+// y-epilogue applied to (K in)(node) for every node of a level with packed
+// element matrices, nv right-hand sides in one launch (vectors at the
+// functors' strides): the two passes, or the one-pass tile kernel where the
+// level has fewer tiles than the solver's threshold (the same sums).  At level
+// 0 of the 10x60x10 super-element model (FP64) the two passes take 9.7 + 5 to 7
+// us a product under ncu against 22 to 30 us for the tile kernel, which waits on
+// 72 scattered loads a thread; a PCG iteration 88.5 -> 82.5 us.
+template <typename T, class In, class Out>
+inline void packed_op(top_solver *s, DevLevel &lv, const In &in, const Out &out, Reduce red, const int *done, int nv)
+{
+    int t0 = 0, nt = 0;
+    coarse_elem_tiles(lv.g, t0, nt);
+    T *W = wbuf<T>(lv);
+    if (W && s->opErr && nt > 0 && nt >= s->coarseTwoPassMin && coarse_elem_occ<T, In>() > 0) {
+        const int64_t wvs = w_alloc_vals(lv.g.cs);
+        const unsigned ctas = (unsigned)std::min<int64_t>(nt, (int64_t)s->numSMs * coarse_elem_occ<T, In>());
+        launch_k(s, coarse_elem_kernel<T, In>, dim3(ctas, (unsigned)nv), kElemThreads, CoarseElem<T>::kSmem, s->st,
+                 in, ks_packed<T>(lv), W, wvs, lv.g, t0, nt, done, s->opErr, s->withholdTile ? 1 : 0);
+        s->withholdTile = false;
+        TOPGPU_COUNT_LAUNCH();
+        launch_k(s, coarse_gather_kernel<T, Out>, dim3((unsigned)lv.g.nbx, (unsigned)lv.g.NZ, (unsigned)nv), kNodeThreads, 0, s->st,
+                 out, W, wvs, lv.g, red, done);
+    } else {
+        dim3 gr = coarse_tile_grid(lv.g); gr.z = (unsigned)nv;
+        launch_k(s, coarse_tile_kernel<T, In, Out>, gr, dim3(kCoarseTileX, 8), 0, s->st, in, out, ks_packed<T>(lv), lv.g, red, done);
+    }
+    TOPGPU_COUNT_LAUNCH();
+}
+}  // namespace topgpu
 
 namespace topgpu {
 // y-epilogue applied to (K_0 in)(node) for every level-0 node, with the
