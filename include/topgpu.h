@@ -83,7 +83,7 @@ int top_assemble_ks_level2(void *Ks, const int32_t *upMap, const void *eleModulu
  * callers that cannot let a library allocate device memory mid-call -- a MEX
  * gateway under MATLAB's gpuArray memory pool, or an application that
  * reserves its memory up front and must avoid the device synchronisation of
- * cudaMalloc/cudaFree.  Its FP64 scratch is a fixed device array (~311 KB per
+ * cudaMalloc/cudaFree.  Its FP64 scratch is a fixed device array (~295 KB per
  * GPU, held until exit); nCh is limited to 64 (TOP_ERR_SHAPE above that).
  * The first call on a device, and the first after its context was replaced
  * (cudaDeviceReset), resolves the array's address (make it before any stream

@@ -2,6 +2,7 @@
 // for sm_100a.  Same arguments, layouts and in-place semantics as the MEX
 // gateways (see include/topgpu.h for the file:line each one replaces).
 #include <cuda_runtime.h>
+#include <algorithm>
 #include <cstdint>
 #include <mutex>
 #include "topgpu_kernels.cuh"
@@ -63,40 +64,32 @@ __global__ void scatter_accum3_kernel(const int32_t *__restrict__ keys, const T 
     for (int c = 0; c < 3; ++c) atomicAdd(&xF[key + c * M], __ldg(&Tmp[i + c * N]));
 }
 
-// Q_s = P_s^T K0 P_s for every child slot (one CTA each): the child-
-// independent part of the level-2 Galerkin product.
+// the element matrix of every regular child, before its modulus
 template <typename T>
 struct K0Child {
     const T *K0;
-    __device__ T operator()(int32_t, int i) const { return K0[i]; }
+    __device__ double operator()(int32_t, int i) const { return double(K0[i]); }
 };
 struct NoSkip { __device__ bool operator()(int32_t) const { return false; } };
 
-// [n x n] identity child map: CTA e of ptkp_kernel then processes slot e only
-__global__ void eye_upmap_kernel(int32_t *up, int n)
-{ int i = blockIdx.x * blockDim.x + threadIdx.x; if (i < n * n) up[i] = (i % (n + 1) == 0) ? 1 : 0; }
-
 // A row of the level-2 GEMM: the moduli of a coarse cell's regular children
 // (0 for void children and for children with fixed DOFs).
+template <typename T>
 struct Level2Row {
-    const int32_t *upMap; const double *E; const int32_t *mapUnique; int64_t nElem; int nCh; int hasFixed;
-    __device__ double operator()(int64_t m, int k) const {
-        if (k >= nCh) return 0.0;
-        const int32_t f1 = upMap[m + (int64_t)k * nElem];
-        if (f1 <= 0) return 0.0;
-        if (hasFixed && mapUnique[f1 - 1] > 0) return 0.0;
-        return E[f1 - 1];
-    }
+    const int32_t *upMap; const T *E; const int32_t *mapUnique; int64_t nElem; int nCh; int hasFixed;
+    __device__ int32_t child(int64_t m, int k) const { return k < nCh ? upMap[m + (int64_t)k * nElem] : 0; }
+    __device__ double value(int32_t f0) const { return double(E[f0]); }
+    __device__ bool regular(int32_t f0) const { return !(hasFixed && mapUnique[f0] > 0); }
 };
 
 template <typename T>
 struct Level2Child {   // K_child of assembleKs_level2_inplace.cu:104-115
     const T *E; const T *K0; const int32_t *mapUnique; const T *uFree; const T *uFixed; int hasFixed;
-    __device__ T operator()(int32_t f0, int i) const {
-        const T mod = E[f0];
+    __device__ double operator()(int32_t f0, int i) const {
+        const double mod = double(E[f0]);
         const int32_t uid0 = hasFixed ? mapUnique[f0] - 1 : -1;
-        if (uid0 >= 0) return uFree[(size_t)uid0 * 576 + i] * mod + uFixed[(size_t)uid0 * 576 + i];
-        return K0[i] * mod;
+        if (uid0 >= 0) return double(uFree[(size_t)uid0 * 576 + i]) * mod + double(uFixed[(size_t)uid0 * 576 + i]);
+        return double(K0[i]) * mod;
     }
 };
 struct RegularChild {  // skip children with fixed DOFs (handled by the GEMM otherwise)
@@ -109,20 +102,20 @@ struct RegularChild {  // skip children with fixed DOFs (handled by the GEMM oth
 template <typename T>
 struct PrevChild {
     const T *KsPrev;
-    __device__ T operator()(int32_t f0, int i) const { return KsPrev[(size_t)f0 * 576 + i]; }
+    __device__ double operator()(int32_t f0, int i) const { return double(KsPrev[(size_t)f0 * 576 + i]); }
 };
 template <typename T>
 struct SuperChild {   // assembleKs_level2_superEle_inplace.cu:113-140
     const T *Ks0; const int32_t *mapUnique; const T *E; const T *uFree; const T *uFixed; int hasFixed;
-    __device__ T operator()(int32_t f0, int i) const {
+    __device__ double operator()(int32_t f0, int i) const {
         const int32_t uid1 = hasFixed ? mapUnique[f0] : 0;
         if (uid1 > 0) {
             const size_t fb = (size_t)(uid1 - 1) * 576 * 64, mb = (size_t)f0 * 64;
-            T acc = T(0);
-            for (int q = 0; q < 64; ++q) acc += uFree[fb + (size_t)q * 576 + i] * E[mb + q];
-            return acc + uFixed[(size_t)(uid1 - 1) * 576 + i];
+            double acc = 0.0;
+            for (int q = 0; q < 64; ++q) acc += double(uFree[fb + (size_t)q * 576 + i]) * double(E[mb + q]);
+            return acc + double(uFixed[(size_t)(uid1 - 1) * 576 + i]);
         }
-        return Ks0[(size_t)f0 * 576 + i];
+        return double(Ks0[(size_t)f0 * 576 + i]);
     }
 };
 
@@ -179,54 +172,108 @@ extern "C" int top_scatter_accum3(const int32_t *keys, const void *Tmp, int64_t 
     return TOP_OK;
 }
 
-namespace topgpu {
+// Single is FP64 inside and rounded on the way out: the SIMT triple products in
+// single took 1410 us for 8192 cells of 64 children, this form 139 us.
 // Level-2 Galerkin assembly in the form Ks = (moduli of regular children) x Q
 // on the FP64 tensor cores, plus the full triple product for children with
-// fixed DOFs.  Shared with the fused solver.  Qscratch: [64 x 576] doubles,
-// zero-filled by the caller; eyeScratch: [nCh x nCh] int32.
-int assemble_level2_f64(double *Ks, const int32_t *upMap, const double *E, const double *K0,
-                        const double *Pch, const int32_t *mapUnique, const double *uFree,
-                        const double *uFixed, int64_t nElem, int nCh, int64_t nUnique,
-                        double *Qscratch, int32_t *eyeScratch, cudaStream_t st,
-                        const int32_t *bndList, int64_t nBnd)
+// fixed DOFs; in FP64 whatever the arrays' type T.  Shared with the fused
+// solver.  Qscratch: [64 x 576] doubles, zero-filled by the caller, or null: each
+// CTA forms the part of Q it multiplies by; numSMs: the current device's.
+namespace {
+// Q_s = P_s^T K0 P_s: the one-child cells of the identity map, written in FP64
+template <typename T>
+__global__ void __launch_bounds__(32) child_q_kernel(double *__restrict__ Q, const T *__restrict__ P, const T *__restrict__ K0)
+{
+    __shared__ double sT[24 * kDmmaLd];
+    const int lane = threadIdx.x, g = lane >> 2, q = lane & 3;
+    double kf[3][6], acc[3][3][2];
+    zero_out(acc);
+    load_child(K0Child<T>{K0}, 0, kf);
+    child_product(P + (size_t)blockIdx.x * 576, kf, sT, acc);
+#pragma unroll
+    for (int I = 0; I < 3; ++I)
+#pragma unroll
+        for (int J = 0; J < 3; ++J)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) Q[(size_t)blockIdx.x * 576 + (8 * I + g) + 24 * (8 * J + 2 * q + h)] = acc[I][J][h];
+}
+template <typename T>
+int assemble_level2(T *Ks, const int32_t *upMap, const T *E, const T *K0, const T *Pch, const int32_t *mapUnique, const T *uFree,
+                    const T *uFixed, int64_t nElem, int nCh, int64_t nUnique, double *Qscratch, cudaStream_t st, int numSMs,
+                    const int32_t *bndList, int64_t nBnd)
 {
     const int hasFixed = (nUnique > 0 && mapUnique && uFree && uFixed) ? 1 : 0;
-    // Q_s = P_s^T K0 P_s, one CTA per child slot
-    if (nCh > 0) {
-        eye_upmap_kernel<<<(nCh * nCh + 255) / 256, 256, 0, st>>>(eyeScratch, nCh);
-        ptkp_f64(st, Qscratch, eyeScratch, nCh, nCh, Pch, K0Child<double>{K0}, NoSkip{}, 0, nullptr, nCh);
-    }
+    const Level2Child<T> child{E, K0, mapUnique, uFree, uFixed, hasFixed};
     if (nElem == 0) return TOP_OK;
     if (nCh <= kGemmK) {
-        cudaFuncSetAttribute(dgemm_k64_kernel<Level2Row>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGemmSmem);
-        // one CTA per row block, looping over the column tiles (the gathered A
-        // tile loaded once instead of once per column tile)
-        dim3 grid((unsigned)((nElem + kGemmBM - 1) / kGemmBM), 1);
-        // B = Qscratch has 64 rows whatever nCh is: the GEMM's K tiles load rows
-        // nCh..63 too and multiply them by the zero A entries that ARow returns
-        // there, so those rows must exist and hold finite values (0 * NaN = NaN)
-        dgemm_k64_kernel<<<grid, 128, kGemmSmem, st>>>(Ks, nElem, 576, 576, Qscratch, 576,
-                                                       Level2Row{upMap, E, mapUnique, nElem, nCh, hasFixed});
+        const Level2Row<T> row{upMap, E, mapUnique, nElem, nCh, hasFixed};
+        const int64_t rb = (nElem + kGemmBM - 1) / kGemmBM;
+        if (Qscratch) {
+            if (nCh > 0) child_q_kernel<T><<<nCh, 32, 0, st>>>(Qscratch, Pch, K0);
+            cudaFuncSetAttribute(dgemm_k64_kernel<T, Level2Row<T>>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGemmSmem);
+            // B = Qscratch has 64 rows whatever nCh is: the GEMM's K tiles load rows
+            // nCh..63 too and multiply them by the zero A entries that ARow returns
+            // there, so those rows must exist and hold finite values (0 * NaN = NaN)
+            dgemm_k64_kernel<<<dim3((unsigned)rb, gemm_k64_split(rb, numSMs)), 128, kGemmSmem, st>>>(Ks, nElem, 576, 576, Qscratch, 576, row);
+        } else {
+            using Kernel = void (*)(T *, int64_t, int, const T *, Level2Row<T>, K0Child<T>);
+            const Kernel kern = gemm_q_kernel<T, Level2Row<T>, K0Child<T>>;
+            cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGemmQSmem);
+            const int64_t perTile = std::max<int64_t>(1, 2 * (int64_t)numSMs / 9);       // two CTAs an SM over the nine column tiles
+            kern<<<dim3((unsigned)std::min(rb, perTile), 9), 128, kGemmQSmem, st>>>(Ks, nElem, nCh, Pch, row, K0Child<T>{K0});
+        }
         // children with fixed DOFs: full triple products, accumulated; only the
         // coarse cells in bndList when the caller knows them (-1: all cells)
         if (hasFixed && nBnd != 0)
-            ptkp_f64(st, Ks, upMap, nElem, nCh, Pch, Level2Child<double>{E, K0, mapUnique, uFree, uFixed, hasFixed},
-                     RegularChild{mapUnique, hasFixed, 1}, 1, nBnd > 0 ? bndList : nullptr, nBnd > 0 ? nBnd : nElem);
+            ptkp(st, numSMs, Ks, upMap, nElem, nCh, Pch, child, RegularChild{mapUnique, hasFixed, 1}, 1,
+                 nBnd > 0 ? bndList : nullptr, nBnd > 0 ? nBnd : nElem);
     } else {
-        ptkp_f64(st, Ks, upMap, nElem, nCh, Pch, Level2Child<double>{E, K0, mapUnique, uFree, uFixed, hasFixed}, NoSkip{}, 0,
-                 nullptr, nElem);
+        ptkp(st, numSMs, Ks, upMap, nElem, nCh, Pch, child, NoSkip{}, 0, nullptr, nElem);
     }
     return cudaGetLastError() == cudaSuccess ? TOP_OK : TOP_ERR_CUDA;
 }
+}  // namespace
+
+namespace topgpu {
+int assemble_level2_f64(double *Ks, const int32_t *upMap, const double *E, const double *K0,
+                        const double *Pch, const int32_t *mapUnique, const double *uFree,
+                        const double *uFixed, int64_t nElem, int nCh, int64_t nUnique,
+                        double *Qscratch, cudaStream_t st, int numSMs, const int32_t *bndList, int64_t nBnd)
+{
+    return assemble_level2<double>(Ks, upMap, E, K0, Pch, mapUnique, uFree, uFixed, nElem, nCh, nUnique, Qscratch, st, numSMs, bndList, nBnd);
+}
 
 int assemble_higher_f64(double *Ks, const int32_t *upMap, const double *KsPrev, const double *Psub,
-                        int64_t nElem, int nSub, cudaStream_t st)
+                        int64_t nElem, int nSub, cudaStream_t st, int numSMs)
 {
     if (nElem == 0) return TOP_OK;
-    ptkp_f64(st, Ks, upMap, nElem, nSub, Psub, PrevChild<double>{KsPrev}, NoSkip{}, 0, nullptr, nElem);
+    ptkp(st, numSMs, Ks, upMap, nElem, nSub, Psub, PrevChild<double>{KsPrev}, NoSkip{}, 0, nullptr, nElem);
     return cudaGetLastError() == cudaSuccess ? TOP_OK : TOP_ERR_CUDA;
 }
 }  // namespace topgpu
+
+namespace {
+// the typed bodies of the gateways (arguments checked, zero elements excluded)
+template <typename T>
+int level2_typed(void *Ks, const int32_t *upMap, const void *E, const void *K0, const void *Pch, const int32_t *mapUnique,
+                 const void *uFree, const void *uFixed, int64_t nElem, int nCh, int64_t nUnique, double *Q, cudaStream_t st)
+{
+    return assemble_level2<T>((T *)Ks, upMap, (const T *)E, (const T *)K0, (const T *)Pch, mapUnique, (const T *)uFree, (const T *)uFixed,
+                              nElem, nCh, nUnique, Q, st, sm_count(), nullptr, -1);
+}
+template <typename T>
+void higher_typed(void *Ks, const int32_t *upMap, const void *KsPrev, const void *Psub, int64_t nElem, int nSub, cudaStream_t st)
+{
+    ptkp(st, sm_count(), (T *)Ks, upMap, nElem, nSub, (const T *)Psub, PrevChild<T>{(const T *)KsPrev}, NoSkip{}, 0, nullptr, nElem);
+}
+template <typename T>
+void super_typed(void *Ks, const int32_t *upMap, const void *Ks0, const void *Psub, const int32_t *mapUnique, const void *E,
+                 const void *uFree, const void *uFixed, int64_t nElem, int nSub, int hasFixed, cudaStream_t st)
+{
+    ptkp(st, sm_count(), (T *)Ks, upMap, nElem, nSub, (const T *)Psub,
+         SuperChild<T>{(const T *)Ks0, mapUnique, (const T *)E, (const T *)uFree, (const T *)uFixed, hasFixed}, NoSkip{}, 0, nullptr, nElem);
+}
+}  // namespace
 
 extern "C" int top_assemble_ks_level2(void *Ks, const int32_t *upMap, const void *eleModulus,
                                       const void *K0, const void *Pch, const int32_t *mapUnique,
@@ -241,28 +288,27 @@ extern "C" int top_assemble_ks_level2(void *Ks, const int32_t *upMap, const void
     if (!Ks || !upMap || !eleModulus || !K0 || !Pch) { set_error("%s:Input null pointer", N); return TOP_ERR_ARGS; }
     const int hasFixed = (nUnique > 0 && mapUnique && uniqueFree && uniqueFixed) ? 1 : 0;
     cudaStream_t st = S(stream);
-    if (dtype == TOP_F64) {
-        struct Scratch {             // stream-ordered frees on every exit of this block
-            void *p = nullptr; cudaStream_t st;
-            explicit Scratch(cudaStream_t q) : st(q) {}
-            ~Scratch() { if (p) cudaFreeAsync(p, st); }
-        } q(st), o(st);
-        const size_t qn = (size_t)576 * (nCh > 64 ? nCh : 64);
-        TOP_CUDA_CHECK(cudaMallocAsync(&q.p, sizeof(double) * qn, st), N);
-        TOP_CUDA_CHECK(cudaMemsetAsync(q.p, 0, sizeof(double) * qn, st), N);
-        TOP_CUDA_CHECK(cudaMallocAsync(&o.p, sizeof(int32_t) * (size_t)nCh * nCh + 4, st), N);
+    struct Scratch {                 // a stream-ordered free on every exit
+        void *p = nullptr; cudaStream_t st;
+        explicit Scratch(cudaStream_t q) : st(q) {}
+        ~Scratch() { if (p) cudaFreeAsync(p, st); }
+    };
+    {
+        Scratch q(st);
+        // One row block of cells in double: no CTA would use its Q tile twice, and
+        // 64 CTAs form Q at once in stream-ordered scratch.  From two row blocks on
+        // (and in single) the CTAs form their own tiles, without an allocation.
+        if (dtype == TOP_F64 && nElem <= kGemmBM) {
+            const size_t qn = (size_t)576 * 64;      // the GEMM's K rows
+            TOP_CUDA_CHECK(cudaMallocAsync(&q.p, sizeof(double) * qn, st), N);
+            TOP_CUDA_CHECK(cudaMemsetAsync(q.p, 0, sizeof(double) * qn, st), N);
+        }
         double *Q = static_cast<double *>(q.p);
-        int32_t *one = static_cast<int32_t *>(o.p);
-        int rc = assemble_level2_f64((double *)Ks, upMap, (const double *)eleModulus, (const double *)K0,
-                                     (const double *)Pch, mapUnique, (const double *)uniqueFree,
-                                     (const double *)uniqueFixed, nElem, nCh, hasFixed ? nUnique : 0, Q, one, st, nullptr, -1);
+        const int64_t nu = hasFixed ? nUnique : 0;
+        const int rc = dtype == TOP_F64
+            ? level2_typed<double>(Ks, upMap, eleModulus, K0, Pch, mapUnique, uniqueFree, uniqueFixed, nElem, nCh, nu, Q, st)
+            : level2_typed<float>(Ks, upMap, eleModulus, K0, Pch, mapUnique, uniqueFree, uniqueFixed, nElem, nCh, nu, Q, st);
         if (rc) { set_error("%s:CUDA launch failed: %s", N, cudaGetErrorString(cudaGetLastError())); return rc; }
-    } else {
-        ptkp_kernel<float><<<(unsigned)nElem, kPtkpThreads, 0, st>>>(
-            (float *)Ks, upMap, nElem, nCh, (const float *)Pch,
-            Level2Child<float>{(const float *)eleModulus, (const float *)K0, mapUnique,
-                               (const float *)uniqueFree, (const float *)uniqueFixed, hasFixed},
-            NoSkip{}, 0, nullptr);
     }
     TOP_CUDA_CHECK(cudaGetLastError(), N);
     TOP_CUDA_CHECK(cudaStreamSynchronize(st), N);   // assembleKs_level2_inplace.cu:272
@@ -279,12 +325,8 @@ extern "C" int top_assemble_ks_higher(void *Ks, const int32_t *upMap, const void
     if (nElem == 0) return TOP_OK;
     if (!Ks || !upMap || !KsPrev || !Psub) { set_error("%s:Input null pointer", N); return TOP_ERR_ARGS; }
     cudaStream_t st = S(stream);
-    if (dtype == TOP_F64)
-        ptkp_f64(st, (double *)Ks, upMap, nElem, nSub, (const double *)Psub, PrevChild<double>{(const double *)KsPrev},
-                 NoSkip{}, 0, nullptr, nElem);
-    else
-        ptkp_kernel<float><<<(unsigned)nElem, kPtkpThreads, 0, st>>>((float *)Ks, upMap, nElem, nSub, (const float *)Psub,
-                                                                     PrevChild<float>{(const float *)KsPrev}, NoSkip{}, 0, nullptr);
+    if (dtype == TOP_F64) higher_typed<double>(Ks, upMap, KsPrev, Psub, nElem, nSub, st);
+    else higher_typed<float>(Ks, upMap, KsPrev, Psub, nElem, nSub, st);
     TOP_CUDA_CHECK(cudaGetLastError(), N);
     TOP_CUDA_CHECK(cudaStreamSynchronize(st), N);   // assembleKs_higherLevel_inplace.cu:209
     return TOP_OK;
@@ -303,15 +345,8 @@ extern "C" int top_assemble_ks_level2_super(void *Ks, const int32_t *upMap, cons
     if (!Ks || !upMap || !Ks0 || !Psub || !eleModulus) { set_error("%s:Input null pointer", N); return TOP_ERR_ARGS; }
     const int hasFixed = (nUnique > 0 && mapUnique && uniqueFree && uniqueFixed) ? 1 : 0;
     cudaStream_t st = S(stream);
-    if (dtype == TOP_F64)
-        ptkp_f64(st, (double *)Ks, upMap, nElem, nSub, (const double *)Psub,
-                 SuperChild<double>{(const double *)Ks0, mapUnique, (const double *)eleModulus,
-                                    (const double *)uniqueFree, (const double *)uniqueFixed, hasFixed}, NoSkip{}, 0, nullptr, nElem);
-    else
-        ptkp_kernel<float><<<(unsigned)nElem, kPtkpThreads, 0, st>>>(
-            (float *)Ks, upMap, nElem, nSub, (const float *)Psub,
-            SuperChild<float>{(const float *)Ks0, mapUnique, (const float *)eleModulus,
-                              (const float *)uniqueFree, (const float *)uniqueFixed, hasFixed}, NoSkip{}, 0, nullptr);
+    if (dtype == TOP_F64) super_typed<double>(Ks, upMap, Ks0, Psub, mapUnique, eleModulus, uniqueFree, uniqueFixed, nElem, nSub, hasFixed, st);
+    else super_typed<float>(Ks, upMap, Ks0, Psub, mapUnique, eleModulus, uniqueFree, uniqueFixed, nElem, nSub, hasFixed, st);
     TOP_CUDA_CHECK(cudaGetLastError(), N);
     TOP_CUDA_CHECK(cudaStreamSynchronize(st), N);   // ..._superEle_inplace.cu:313
     return TOP_OK;
@@ -326,9 +361,9 @@ extern "C" int top_assemble_ks_level2_super(void *Ks, const int32_t *upMap, cons
 // applications that reserve their memory once up front and must not pay the
 // implicit device synchronisation of cudaMalloc/cudaFree inside an
 // optimisation loop.  This entry point takes its scratch (the child matrices
-// Q_s = P_s' K0 P_s and the slot map of the level-2 Galerkin GEMM) from the
-// fixed device arrays below, which every GPU that loads the library holds
-// until the process exits (about 311 KB per device).
+// Q_s = P_s' K0 P_s of the level-2 Galerkin GEMM) from the
+// fixed device array below, which every GPU that loads the library holds
+// until the process exits (about 295 KB per device).
 //
 // Limits and behaviour:
 //  * at most kNoAllocMaxChildren (64) children per coarse element -- the
@@ -345,14 +380,13 @@ namespace {
 constexpr int kNoAllocMaxChildren = 64;
 constexpr int kNoAllocMaxDevices = 64;
 static __device__ __align__(256) double g_noalloc_Q[576 * kNoAllocMaxChildren];
-static __device__ __align__(256) int32_t g_noalloc_eye[kNoAllocMaxChildren * kNoAllocMaxChildren];
 
 // The resolved addresses are valid for one context of one device: a device
 // reset unloads the module and the next context may place the arrays
 // elsewhere, so the cache is keyed on (device, current context).  The context
 // handle comes from the driver's cuCtxGetCurrent, looked up through the
 // runtime (no link against libcuda).
-struct NoAllocScratch { double *Q = nullptr; int32_t *eye = nullptr; void *ctx = nullptr; };
+struct NoAllocScratch { double *Q = nullptr; void *ctx = nullptr; };
 std::mutex g_noalloc_mu;
 NoAllocScratch g_noalloc_dev[kNoAllocMaxDevices];
 bool g_noalloc_ready[kNoAllocMaxDevices] = {};
@@ -386,7 +420,6 @@ int noalloc_scratch(NoAllocScratch *out, const char *N)
     if (!g_noalloc_ready[dev] || g_noalloc_dev[dev].ctx != ctx) {
         NoAllocScratch s;
         TOP_CUDA_CHECK(cudaGetSymbolAddress((void **)&s.Q, g_noalloc_Q), N);
-        TOP_CUDA_CHECK(cudaGetSymbolAddress((void **)&s.eye, g_noalloc_eye), N);
         s.ctx = ctx;
         g_noalloc_dev[dev] = s;
         g_noalloc_ready[dev] = true;
@@ -413,25 +446,18 @@ extern "C" int top_assemble_ks_level2_noalloc(void *Ks, const int32_t *upMap, co
     if (!Ks || !upMap || !eleModulus || !K0 || !Pch) { set_error("%s:Input null pointer", N); return TOP_ERR_ARGS; }
     const int hasFixed = (nUnique > 0 && mapUnique && uniqueFree && uniqueFixed) ? 1 : 0;
     cudaStream_t st = S(stream);
-    if (dtype == TOP_F64) {
-        NoAllocScratch sc;
-        int rc = noalloc_scratch(&sc, N);
-        if (rc) return rc;
-        // the GEMM loads all 64 rows of Q and multiplies rows nCh..63 by zero:
-        // clear them all, so that no value left by an earlier call (NaN or Inf
-        // included) reaches this call's result
-        TOP_CUDA_CHECK(cudaMemsetAsync(sc.Q, 0, sizeof(double) * 576 * kNoAllocMaxChildren, st), N);
-        rc = assemble_level2_f64((double *)Ks, upMap, (const double *)eleModulus, (const double *)K0,
-                                 (const double *)Pch, mapUnique, (const double *)uniqueFree,
-                                 (const double *)uniqueFixed, nElem, nCh, hasFixed ? nUnique : 0, sc.Q, sc.eye, st, nullptr, -1);
-        if (rc) { set_error("%s:CUDA launch failed: %s", N, cudaGetErrorString(cudaGetLastError())); return rc; }
-    } else {
-        ptkp_kernel<float><<<(unsigned)nElem, kPtkpThreads, 0, st>>>(
-            (float *)Ks, upMap, nElem, nCh, (const float *)Pch,
-            Level2Child<float>{(const float *)eleModulus, (const float *)K0, mapUnique,
-                               (const float *)uniqueFree, (const float *)uniqueFixed, hasFixed},
-            NoSkip{}, 0, nullptr);
-    }
+    NoAllocScratch sc;
+    int rc = noalloc_scratch(&sc, N);
+    if (rc) return rc;
+    // the GEMM loads all 64 rows of Q and multiplies rows nCh..63 by zero:
+    // clear them all, so that no value left by an earlier call (NaN or Inf
+    // included) reaches this call's result
+    TOP_CUDA_CHECK(cudaMemsetAsync(sc.Q, 0, sizeof(double) * 576 * kNoAllocMaxChildren, st), N);
+    const int64_t nu = hasFixed ? nUnique : 0;
+    rc = dtype == TOP_F64
+        ? level2_typed<double>(Ks, upMap, eleModulus, K0, Pch, mapUnique, uniqueFree, uniqueFixed, nElem, nCh, nu, sc.Q, st)
+        : level2_typed<float>(Ks, upMap, eleModulus, K0, Pch, mapUnique, uniqueFree, uniqueFixed, nElem, nCh, nu, sc.Q, st);
+    if (rc) { set_error("%s:CUDA launch failed: %s", N, cudaGetErrorString(cudaGetLastError())); return rc; }
     TOP_CUDA_CHECK(cudaGetLastError(), N);
     TOP_CUDA_CHECK(cudaStreamSynchronize(st), N);
     return TOP_OK;

@@ -23,12 +23,9 @@ namespace topgpu {
 int assemble_level2_f64(double *Ks, const int32_t *upMap, const double *E, const double *K0,
                         const double *Pch, const int32_t *mapUnique, const double *uFree,
                         const double *uFixed, int64_t nElem, int nCh, int64_t nUnique,
-                        double *Qscratch, int32_t *eyeScratch, cudaStream_t st,
-                        const int32_t *bndList, int64_t nBnd);
+                        double *Qscratch, cudaStream_t st, int numSMs, const int32_t *bndList, int64_t nBnd);
 int assemble_higher_f64(double *Ks, const int32_t *upMap, const double *KsPrev, const double *Psub,
-                        int64_t nElem, int nSub, cudaStream_t st);
-
-
+                        int64_t nElem, int nSub, cudaStream_t st, int numSMs);
 
 // ---------------------------------------------------------------------------
 // small kernels
@@ -991,8 +988,7 @@ extern "C" int top_solver_create(const top_mesh *mesh, const top_solver_params *
     s->P4 = s->dalloc<double>((size_t)576 * 64);
     s->P2 = s->dalloc<double>((size_t)576 * 8);
     s->Qs = s->dalloc<double>((size_t)576 * 64);
-    s->eye = s->dalloc<int32_t>(64 * 64 + 4);
-    if (!s->KeDev || !s->Ec || !s->Eg64 || !s->Eg32 || !s->mapUnique || !s->uFree || !s->uFixed || !s->P4 || !s->P2 || !s->Qs || !s->eye)
+    if (!s->KeDev || !s->Ec || !s->Eg64 || !s->Eg32 || !s->mapUnique || !s->uFree || !s->uFixed || !s->P4 || !s->P2 || !s->Qs)
         return fail("out of device memory");
     cudaMemcpy(s->KeDev, M0.Ke, sizeof(double) * 576, cudaMemcpyHostToDevice);
     if (s->nL > 1) {   // coarse level-1 cells that own a child with fixed DOFs
@@ -1518,12 +1514,12 @@ extern "C" int top_solver_assemble(top_solver *s)
         int rc;
         if (s->super)    // P_s' K_mat(child) P_s, K_mat with the boundary override (superEle_inplace.cu:70-173)
             rc = assemble_higher_f64(d.KsC, d.upMap, s->L[l - 1].KsC, d.span == 4 ? s->P4 : s->P2, d.Ne,
-                                     d.span * d.span * d.span, st);
+                                     d.span * d.span * d.span, st, s->numSMs);
         else if (l == 1)
             rc = assemble_level2_f64(d.KsC, d.upMap, s->Ec, s->KeDev, s->P4, s->mapUnique, s->uFree, s->uFixed,
-                                     d.Ne, 64, s->nU, s->Qs, s->eye, st, s->bndList, s->nBnd);
+                                     d.Ne, 64, s->nU, s->Qs, st, s->numSMs, s->bndList, s->nBnd);
         else
-            rc = assemble_higher_f64(d.KsC, d.upMap, s->L[l - 1].KsC, s->P2, d.Ne, 8, st);
+            rc = assemble_higher_f64(d.KsC, d.upMap, s->L[l - 1].KsC, s->P2, d.Ne, 8, st, s->numSMs);
         if (rc) { set_error("top_solver_assemble: Galerkin kernel failed"); return rc; }
         if (l < s->nL - 1) {
             pack_ks_kernel<<<(unsigned)((d.Ne + kPackE - 1) / kPackE), 256, 0, st>>>(d.KsC, d.eleGrid, d.Ne, d.KsP64, d.KsP32, d.g.cs);

@@ -105,7 +105,7 @@ struct top_solver {
     double *KeDev = nullptr, *P4 = nullptr, *P2 = nullptr;
     double *Ec = nullptr, *Eg64 = nullptr; float *Eg32 = nullptr;
     int32_t *mapUnique = nullptr; double *uFree = nullptr, *uFixed = nullptr; int64_t nU = 0;
-    double *Qs = nullptr; int32_t *eye = nullptr;
+    double *Qs = nullptr;
     int32_t *bndList = nullptr; int64_t nBnd = 0;   // level-1 cells with fixed-DOF children
     double *x = nullptr, *r = nullptr, *z = nullptr, *pv = nullptr, *v = nullptr, *tmp = nullptr;
     float *z32 = nullptr;            // FP32 preconditioned residual of the mixed path
