@@ -8,6 +8,7 @@
 #include <cmath>
 #include <cstring>
 #include <type_traits>
+#include <vector>
 #include "topgpu_solver_impl.cuh"
 #include "topgpu_stage.cuh"
 
@@ -165,7 +166,7 @@ void l0_op(top_solver *s, const In &in, const Out &out, Reduce red, const int *d
 #define TOPGPU_LAUNCH_SHAPE(A, B)                                                                             \
         if (k.ty == A && k.tx == B)                                                                           \
             launch_k(s, l0d_kernel<T, A, B, In, Out>, dim3(l0w_ctas<T, A, B, In, Out, 3>(s, k), K), A * B, 0, s->st,   \
-                walshparam<T>(s), in, out, egrid<T>(s), lv.flags, k.mask, lv.g, T(s->p.E0), red, done);
+                walshparam<T>(s), in, out, egrid<T>(s), lv.flags, k.mask, lv.g, T(s->p.E0), red, done, k.rng);
         TOPGPU_WALSH_SHAPES(TOPGPU_LAUNCH_SHAPE)
 #undef TOPGPU_LAUNCH_SHAPE
     } else if (k.kind == 5) {        // FP32 only: tensor cores, 16 x 8 element columns
@@ -183,7 +184,7 @@ void l0_op(top_solver *s, const In &in, const Out &out, Reduce red, const int *d
 #undef TOPGPU_LAUNCH_SHAPE
         } else if constexpr (sizeof(T) == 4) {   // another operand type: the direct-load kind, same tile shape
             launch_k(s, l0d_kernel<T, 16, 8, In, Out>, dim3(l0w_ctas<T, 16, 8, In, Out, 3>(s, s->l0kFallback), K), 128, 0, s->st,
-                walshparam<T>(s), in, out, egrid<T>(s), lv.flags, s->l0kFallback.mask, lv.g, T(s->p.E0), red, done);
+                walshparam<T>(s), in, out, egrid<T>(s), lv.flags, s->l0kFallback.mask, lv.g, T(s->p.E0), red, done, (const int2 *)nullptr);
         }
     } else if (k.kind == 4) {        // FP32 only, as kind 2
         if constexpr (sizeof(T) == 4) {
@@ -310,6 +311,26 @@ int tc_selftest(top_solver *s, const top_solver::L0Kernel &cand)
 }
 }  // namespace
 
+// kind 3's ranges of active layers (kept null where no tile leaves any out)
+static int l0_active_ranges(top_solver *s, top_solver::L0Kernel &k, int ty, int tx)
+{
+    const Geom &g = s->L[0].g;
+    const int tiles = walsh_tiles(g, ty, tx);
+    int2 *rng = nullptr;
+    if (cudaMalloc(&rng, sizeof(int2) * (size_t)tiles) != cudaSuccess) return TOP_ERR_NOMEM;
+#define TOPGPU_RANGE_SHAPE(A, B) if (ty == A && tx == B) walsh_range_kernel<A, B><<<tiles, 256, 0, s->st>>>(s->L[0].flags, g, rng);
+    TOPGPU_WALSH_SHAPES(TOPGPU_RANGE_SHAPE)
+#undef TOPGPU_RANGE_SHAPE
+    TOPGPU_COUNT_LAUNCH();
+    std::vector<int2> r((size_t)tiles);
+    if (cudaMemcpyAsync(r.data(), rng, sizeof(int2) * r.size(), cudaMemcpyDeviceToHost, s->st) != cudaSuccess ||
+        cudaStreamSynchronize(s->st) != cudaSuccess) { cudaFree(rng); return TOP_ERR_CUDA; }
+    for (const int2 &t : r)
+        if (t.x > 0 || t.y < g.NZ) { k.rng = rng; return TOP_OK; }
+    cudaFree(rng);
+    return TOP_OK;
+}
+
 int set_l0_kernel(top_solver *s, int p, int kind, int ty, int tx, int ctas)
 {
     top_solver::L0Kernel &k = s->l0k[p];
@@ -357,6 +378,11 @@ int set_l0_kernel(top_solver *s, int p, int kind, int ty, int tx, int ctas)
         const int rc = tc_selftest(s, cand);
         if (rc != TOP_OK) return rc;
         if (s->stageErr) { set_error("level-0 kernel kind 6: tensor map encoding failed"); return TOP_ERR_CUDA; }
+    }
+    if (k.rng) { cudaFree(k.rng); k.rng = nullptr; }
+    if (kind == 3) {
+        const int rc = l0_active_ranges(s, k, ty, tx);
+        if (rc != TOP_OK) { k.kind = 0; ++s->opGen; return rc; }
     }
     k.kind = kind; k.ty = ty; k.tx = tx; k.ctas = ctas;
     ++s->opGen;

@@ -73,7 +73,12 @@ struct top_solver {
     // paired with TMA-staged node layers (FP32; tiles of 2 ty x tx), on
     // ctas CTAs (0: as many as fit at once); per precision, set by
     // top_solver_set_l0_kernel or the autotuner
-    struct L0Kernel { int kind = 0, ty = 16, tx = 16, ctas = 0; uint8_t *mask = nullptr; };
+    struct L0Kernel {
+        int kind = 0, ty = 16, tx = 16, ctas = 0; uint8_t *mask = nullptr;
+        int2 *rng = nullptr;         // kind 3: each tile's range of layers with active nodes (null: all of them)
+    };
+    // chunks of the level-0 vectors that the PCG vector kernels visit (ChunkList; null: all of them)
+    int32_t *chunks = nullptr; int nChunks = 0;
     int numSMs = 148;
     L0Kernel l0k[2];                 // [0] FP64, [1] FP32
     L0Kernel l0kFallback;            // kind 6 with a converting operand: the direct-load kind, 16 x 8
