@@ -150,6 +150,23 @@ dgemm_tile_kernel(double *C, int64_t ldc, const double *A, int64_t lda, const do
     });
 }
 
+// A^-1 = W^T W as packed lower tiles: tile (I, J), J <= I, at index I (I + 1) / 2 + J,
+// 64 x 64 column-major, zero past row or column n (the diagonal tiles whole)
+__global__ void __launch_bounds__(kTileThreads)
+wtw_packed_kernel(double *__restrict__ P, const double *__restrict__ W, int64_t n)
+{
+    __shared__ double sm[tile_smem_vals<true, true>];
+    const int i0 = blockIdx.x * kTileB, j0 = blockIdx.y * kTileB;
+    if (j0 > i0) return;
+    double acc[4][4][2];
+    zero_acc(acc);
+    dmma_tile<true, true>([&](int r, int k) { const int i = i0 + r; return i < n ? W[k + n * i] : 0.0; },
+                          [&](int r, int k) { const int j = j0 + r; return j < n ? W[k + n * j] : 0.0; },
+                          i0, (int)n, acc, sm, NoFold{});
+    double *T = P + ((int64_t)blockIdx.x * (blockIdx.x + 1) / 2 + blockIdx.y) * kTileB * kTileB;
+    each_out(acc, [&](int r, int c, double v) { T[c * kTileB + r] = v; });
+}
+
 // One level of the bottom-up block inversion of a lower-triangular L (n x n):
 // node z covers rows [r0, r0 + 2 hs), r0 = 2 hs z, split at rh = r0 + hs; its
 // two products, over blockIdx.z:

@@ -1038,20 +1038,10 @@ restrict_xz_kernel(const T *__restrict__ t, int NXf, int NZf, T *__restrict__ rc
 // eight loads of the row in flight, the warps reduce by shuffles and thread
 // 0 adds the warp sums in a fixed order and returns them in out.
 constexpr int kCoarsestThreads = 256;
-// coarsest right-hand sides gathered in compact order (k at cr + k n)
-struct CompactRhs {
-    const double *cr; int64_t n;
-    __device__ __forceinline__ double operator()(int k, int64_t j) const { return cr[k * n + j]; }
-};
-// ... or staged in shared memory ([k - v0][n] for the group starting at v0)
-struct StagedRhs {
-    const double *s; int64_t n; int v0;
-    __device__ __forceinline__ double operator()(int k, int64_t j) const { return s[(k - v0) * n + j]; }
-};
-// ... or read from the level's grid vector (k at r + k vs)
-template <typename T> struct GridRhs {
-    const T *r; int64_t vs, cs; const int32_t *nodeGrid;
-    __device__ __forceinline__ double operator()(int k, int64_t j) const { return double(r[k * vs + (j % 3) * cs + nodeGrid[j / 3]]); }
+// coarsest right-hand sides in compact order (k at cr + k n)
+template <typename T> struct CompactRhs {
+    const T *cr; int64_t n;
+    __device__ __forceinline__ double operator()(int k, int64_t j) const { return double(cr[k * n + j]); }
 };
 template <class Rhs>
 __device__ __forceinline__ void coarsest_row(const double *__restrict__ a, const Rhs &cr, int64_t n, int v0,

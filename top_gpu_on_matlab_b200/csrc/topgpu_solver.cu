@@ -205,18 +205,17 @@ coarsest_assemble_kernel(const double *__restrict__ KsC, const int32_t *__restri
 // ---- coarsest level ----
 // coarsest solve: x_grid = Ainv * r
 // one CTA per row of A^-1, every right-hand side (up to four per pass over the
-// row), read from the level's grid vector r in compact order
+// row), read from their compact copy r, which the restriction into the level
+// writes (gathered from the grid into every CTA's shared memory, the mixed
+// V-cycle's form before, 1386 rows took 17.6 us)
 template <typename T>
 __global__ void __launch_bounds__(kCoarsestThreads)
 coarsest_gemv_kernel(const double *__restrict__ Ainv, const T *__restrict__ r, int64_t n,
                      T *__restrict__ x, Geom g, const int32_t *__restrict__ nodeGrid,
-                     const int *__restrict__ done0, int64_t vs, int nv, int staged)
+                     const int *__restrict__ done0, int64_t vs, int nv)
 {
-    // staged 1: the right-hand sides gathered from the grid into shared memory;
-    // 2 (FP64): read from their compact copy r; 0: read from the grid per term
     pdl_enter();
     __shared__ double red[kCoarsestThreads / 32][4];
-    extern __shared__ double rstage[];           // staged: the right-hand sides [4][n]
     const int64_t row = blockIdx.x;
     for (int v0 = 0; v0 < nv; v0 += 4) {
         bool act[4];
@@ -229,40 +228,147 @@ coarsest_gemv_kernel(const double *__restrict__ Ainv, const T *__restrict__ r, i
         }
         if (!any) continue;                      // uniform in the CTA
         double out[4];
-        if (staged == 1) {
-            // the right-hand sides into shared memory first (all the node-map
-            // loads of a thread, then all its value loads), then the same sums
-            __syncthreads();                     // the previous group's reads are done
-            for (int64_t j0 = threadIdx.x; j0 < n; j0 += (int64_t)kCoarsestThreads * 4) {
-                int32_t slot[4];
-#pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    const int64_t j = j0 + (int64_t)kCoarsestThreads * u;
-                    slot[u] = j < n ? nodeGrid[j / 3] : 0;
-                }
-#pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    const int64_t j = j0 + (int64_t)kCoarsestThreads * u;
-                    if (j >= n) break;
-#pragma unroll
-                    for (int q = 0; q < 4; ++q)
-                        if (act[q]) rstage[q * n + j] = double(r[(v0 + q) * vs + (j % 3) * g.cs + slot[u]]);
-                }
-            }
-            __syncthreads();
-            coarsest_row(Ainv + n * row, StagedRhs{rstage, n, v0}, n, v0, act, red, out);
-        } else if (staged == 2) {
-            // FP64: r is the compact copy the restriction wrote ([k][n], the same values)
-            if constexpr (sizeof(T) == 8)
-                coarsest_row(Ainv + n * row, CompactRhs{reinterpret_cast<const double *>(r), n}, n, v0, act, red, out);
-        } else {
-            coarsest_row(Ainv + n * row, GridRhs<T>{r, vs, g.cs, nodeGrid}, n, v0, act, red, out);
-        }
+        coarsest_row(Ainv + n * row, CompactRhs<T>{r, n}, n, v0, act, red, out);
         if (threadIdx.x == 0)
 #pragma unroll
             for (int q = 0; q < 4; ++q)
                 if (act[q]) x[(v0 + q) * vs + (row % 3) * g.cs + nodeGrid[row / 3]] = T(out[q]);
     }
+}
+// The same product on large coarsest levels, bound by the bytes of A^-1: it is
+// symmetric, so its packed lower tiles (half the bytes) serve both y_I += A_IJ x_J
+// and y_J += A_IJ^T x_I.  A persistent CTA brings its 32 KB tiles into shared memory
+// by bulk copies, two in flight (bounded waits: on a give-up the error flag goes
+// up); thread (r, h) sums half h of row r, then half h of column r, walking the
+// column from its own row on so that a half-warp's reads fall in distinct banks.
+// Each tile's two partial vectors go to part[rhs][tile][2][64]; sym_sum_kernel
+// adds a row's over the tiles in order (deterministic).  Measured (FP64 PCG,
+// iteration, whole -> packed): 4131 DOFs 216.7 -> 195.2 us, 2496 154.1 -> 141.8,
+// 1617 120.4 -> 117.2, 675 84.0 -> 86.4: from 2000 DOFs on.
+constexpr int64_t kSymMinDofs = 2000;
+constexpr int kSymT = kTileB, kSymThreads = 2 * kSymT;
+constexpr uint32_t kSymTileBytes = sizeof(double) * kSymT * kSymT;
+constexpr size_t kSymSmem = 2 * kSymTileBytes + sizeof(double) * (4 * 2 * kSymT + 2 * kSymT) + 16;
+__device__ __forceinline__ void sym_tile(int t, int &I, int &J)
+{
+    I = (int)((sqrtf(8.0f * (float)t + 1.0f) - 1.0f) * 0.5f);
+    while ((I + 1) * (I + 2) / 2 <= t) ++I;
+    while (I * (I + 1) / 2 > t) --I;
+    J = t - I * (I + 1) / 2;
+}
+template <typename T>
+__global__ void __launch_bounds__(kSymThreads)
+sym_gemv_kernel(const double *__restrict__ P, const T *__restrict__ rc, int64_t n, int tiles, double *__restrict__ part,
+                const int *__restrict__ done0, int nv, int *err)
+{
+    pdl_enter();
+    extern __shared__ __align__(128) unsigned char sym_smem[];
+    double *buf = reinterpret_cast<double *>(sym_smem);                 // two tiles
+    double *xs = buf + 2 * kSymT * kSymT;                               // [4][x_I, x_J]
+    double *half = xs + 4 * 2 * kSymT;                                  // [row, column][64]
+    const uint32_t bar = bulk::smem_addr(half + 2 * kSymT);
+    const int t = threadIdx.x, r = t & (kSymT - 1), h = t >> 6;
+    if (t == 0) {
+        bulk::bar_init(bar, 1u);
+        bulk::bar_init(bar + 8, 1u);
+        bulk::fence_init();
+    }
+    __syncthreads();
+    int k = 0;                               // tiles waited for, over all groups of right-hand sides
+    auto issue = [&](int tile, int slot) {
+        if (t != 0 || tile >= tiles) return;
+        bulk::arrive_expect(bar + 8 * slot, kSymTileBytes);
+        bulk::copy(bulk::smem_addr(buf + slot * kSymT * kSymT), P + (int64_t)tile * kSymT * kSymT, kSymTileBytes, bar + 8 * slot);
+    };
+    for (int v0 = 0; v0 < nv; v0 += 4) {
+        bool act[4];
+        bool any = false;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int *d = done_of(done0, v0 + q);
+            act[q] = v0 + q < nv && !(d && *d);
+            any = any || act[q];
+        }
+        if (!any) continue;                  // uniform in the CTA
+        int tile = blockIdx.x, I, J;
+        issue(tile, k & 1);
+        issue(tile + (int)gridDim.x, (k + 1) & 1);
+        double xr[4];                        // x_I (h = 0) or x_J (h = 1) of the next tile
+        auto load_x = [&](int tl) {
+            if (tl >= tiles) return;
+            int a, b;
+            sym_tile(tl, a, b);
+            const int64_t j = (int64_t)(h ? b : a) * kSymT + r;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) xr[q] = act[q] && j < n ? double(rc[(v0 + q) * n + j]) : 0.0;
+        };
+        load_x(tile);
+        for (; tile < tiles; tile += gridDim.x, ++k) {
+            sym_tile(tile, I, J);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) xs[(2 * q + h) * kSymT + r] = xr[q];
+            load_x(tile + (int)gridDim.x);
+            const bool got = bulk::wait(bar + 8 * (k & 1), (uint32_t)(k >> 1) & 1u);
+            if (!__syncthreads_and(got)) {   // uniform: every thread leaves
+                if (t == 0) {
+                    atomicExch(err, 1);
+                    // this tile and the next may still be landing: wait for them (bounded)
+                    (void)bulk::wait(bar + 8 * (k & 1), (uint32_t)(k >> 1) & 1u);
+                    if (tile + (int)gridDim.x < tiles) (void)bulk::wait(bar + 8 * ((k + 1) & 1), (uint32_t)((k + 1) >> 1) & 1u);
+                }
+                return;
+            }
+            const double *A = buf + (k & 1) * kSymT * kSymT;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                if (!act[q]) continue;
+                const double *xI = xs + 2 * q * kSymT, *xJ = xI + kSymT;
+                double row = 0.0, col = 0.0;
+#pragma unroll 8
+                for (int c = 32 * h; c < 32 * h + 32; ++c) row = fma(A[c * kSymT + r], xJ[c], row);
+                if (I != J)
+#pragma unroll 8
+                    for (int u = 0; u < 32; ++u) {
+                        const int m = 32 * h + ((u + r) & 31);
+                        col = fma(A[r * kSymT + m], xI[m], col);
+                    }
+                if (h) { half[r] = row; half[kSymT + r] = col; }
+                __syncthreads();
+                if (!h) {
+                    double *o = part + ((int64_t)(v0 + q) * tiles + tile) * 2 * kSymT;
+                    o[r] = row + half[r];
+                    o[kSymT + r] = col + half[kSymT + r];
+                }
+                __syncthreads();             // half (and, after the last q, xs and the tile) are free
+            }
+            issue(tile + 2 * (int)gridDim.x, k & 1);
+        }
+    }
+}
+// y of 64 rows: their partial vectors over the tiles, in tile order, four
+// interleaved sums a row added in order
+template <typename T>
+__global__ void __launch_bounds__(4 * kSymT)
+sym_sum_kernel(const double *__restrict__ part, int64_t n, int tiles, T *__restrict__ x, Geom g, const int32_t *__restrict__ nodeGrid,
+               const int *__restrict__ done0, int64_t vs)
+{
+    pdl_enter();
+    const int vk = blockIdx.y;
+    const int *done = done_of(done0, vk);
+    if (done && *done) return;
+    __shared__ double red[4][kSymT];
+    const int I = blockIdx.x, nt = gridDim.x, r = threadIdx.x & (kSymT - 1), w = threadIdx.x >> 6;
+    const double *p = part + (int64_t)vk * tiles * 2 * kSymT;
+    double s = 0.0;
+#pragma unroll 4
+    for (int m = w; m < nt; m += 4) {
+        const int64_t tile = m <= I ? (int64_t)I * (I + 1) / 2 + m : (int64_t)m * (m + 1) / 2 + I;
+        s += p[tile * 2 * kSymT + (m <= I ? 0 : kSymT) + r];
+    }
+    red[w][r] = s;
+    __syncthreads();
+    const int64_t row = (int64_t)I * kSymT + r;
+    if (w == 0 && row < n) x[vk * vs + (row % 3) * g.cs + nodeGrid[row / 3]] = T(red[0][r] + red[1][r] + red[2][r] + red[3][r]);
 }
 
 // ---- the V-cycle's condensed tail: t = M r on one level's active DOFs ----
@@ -605,21 +711,11 @@ __global__ void compliance_kmat_kernel(const double *__restrict__ Kc, const doub
 
 using namespace topgpu;
 
-// the V-cycle's condensed tail (defined with the coarsest solve below)
+// A^-1 = W^T W as a whole matrix in s->Ainv (defined with the coarsest solve below)
+void whole_inverse(top_solver *s, cudaStream_t st);
+// the V-cycle's condensed tail (likewise)
 bool tail_on(const top_solver *s);
 int build_tail(top_solver *s, cudaStream_t st);
-
-// dynamic shared memory of a GEMV that stages its right-hand sides (up to
-// four groups of n FP64 values, at most 96 KB), 0 beyond: those read them
-// from the grid
-template <typename T>
-size_t gemv_stage_bytes(int64_t n, int nv)
-{
-    constexpr size_t kMax = 96 * 1024;
-    static const bool attr = cudaFuncSetAttribute(coarsest_gemv_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMax) == cudaSuccess;
-    const size_t b = sizeof(double) * (size_t)(nv < 4 ? nv : 4) * (size_t)n;
-    return (attr && b <= kMax) ? b : 0;
-}
 
 namespace {
 
@@ -686,8 +782,8 @@ void coarse_elem_setup()
     (void)coarse_elem_occ<double, JacobiIn<double, double>>();
     (void)coarse_elem_occ<double, VecIn<double, double>>();
     (void)coarse_elem_occ<float, VecIn<float, double>>();
-    (void)gemv_stage_bytes<float>(1, 1);
-    (void)gemv_stage_bytes<double>(1, 1);
+    (void)cudaFuncSetAttribute(sym_gemv_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSymSmem);
+    (void)cudaFuncSetAttribute(sym_gemv_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSymSmem);
 }
 
 // y-epilogue applied to (K_level in)(node) for every node of a coarse level;
@@ -779,8 +875,8 @@ void vcycle(top_solver *s, const TR *r0, TZ *z0, double *zr, const int *done, in
     // in the precision of the solver's V-cycle
     const bool tailT = sizeof(T) == (s->p.precision == TOP_PREC_MIXED ? 4u : 8u);
     const int tl = (!persist && tailT && s->tailReady && tail_on(s)) ? s->tailL : 0;
-    // FP64 coarsest GEMV reading the compact copy of its right-hand sides
-    const bool cmpC = sizeof(T) == 8 && !persist && !tl && nv <= s->kMax;
+    // the coarsest GEMV reads the compact copy of its right-hand sides (s->cr holds it in either type)
+    const bool cmpC = !persist && !tl;
     if (!z1Ready) {
         DevLevel &l0 = s->L[0];
         const int64_t n0 = lvs(l0), M = kMargin;
@@ -798,8 +894,7 @@ void vcycle(top_solver *s, const TR *r0, TZ *z0, double *zr, const int *done, in
         else
             coarse_op<T>(s, l, JacobiIn<T, T>{vr<T>(lv), invd<T>(lv), lv.g.cs, omega, vs}, ResidOut<T, T, T>{vr<T>(lv), d, lv.g.cs, vs},
                          none, done, nv);
-        // into the tail's level: r also in compact order, the GEMV's operand;
-        // likewise (FP64) into the coarsest level for its GEMV
+        // into the tail's or the coarsest level: r also in compact order, the GEMV's operand
         if (tl && l + 1 == tl)
             restrict_op<T>(s, l, d, vr<T>(lc), done, nv, static_cast<T *>(s->tailR), s->tailNodeCompact[0], s->tailLd);
         else if (cmpC && l + 1 == nL - 1)
@@ -841,11 +936,19 @@ void vcycle(top_solver *s, const TR *r0, TZ *z0, double *zr, const int *done, in
         cudaLaunchKernelEx(&cfg, coarse_vcycle_kernel<T>, A, done);
         TOPGPU_COUNT_LAUNCH();
     } else {
-        // coarsest direct solve, FP64 (the right-hand side read from the grid by the product)
-        const size_t sm = cmpC ? 0 : gemv_stage_bytes<T>(n, nv);
-        launch_k(s, coarsest_gemv_kernel<T>, (unsigned)n, kCoarsestThreads, sm, s->st, s->Ainv,
-                 cmpC ? reinterpret_cast<const T *>(s->cr) : (const T *)vr<T>(lc), n, vt<T>(lc), lc.g,
-                 lc.nodeGrid, done, lvs(lc), nv, cmpC ? 2 : (sm ? 1 : 0));
+        // coarsest direct solve, FP64
+        const T *rc = reinterpret_cast<const T *>(s->cr);
+        if (s->symPart) {
+            const int nt = (int)((n + kSymT - 1) / kSymT), tiles = nt * (nt + 1) / 2;
+            launch_k(s, sym_gemv_kernel<T>, (unsigned)std::min(tiles, 3 * s->numSMs), kSymThreads, kSymSmem, s->st,
+                     (const double *)s->Ac, rc, n, tiles, s->symPart, done, nv, s->opErr);
+            TOPGPU_COUNT_LAUNCH();
+            launch_k(s, sym_sum_kernel<T>, dim3((unsigned)nt, K), 4 * kSymT, 0, s->st,
+                     (const double *)s->symPart, n, tiles, vt<T>(lc), lc.g, lc.nodeGrid, done, lvs(lc));
+        } else {
+            launch_k(s, coarsest_gemv_kernel<T>, (unsigned)n, kCoarsestThreads, 0, s->st, s->Ainv, rc, n, vt<T>(lc), lc.g,
+                     lc.nodeGrid, done, lvs(lc), nv);
+        }
         TOPGPU_COUNT_LAUNCH();
     }
     // interpolation leg
@@ -1165,6 +1268,11 @@ extern "C" int top_solver_create(const top_mesh *mesh, const top_solver_params *
         s->Wc = s->dalloc<double>((size_t)s->nC * s->nC);
         s->Dc = s->dalloc<double>((size_t)((s->nC + kDb - 1) / kDb) * kDb * kDb);
         s->cr = s->dalloc<double>((size_t)s->nC * s->kMax);
+        if (s->nC > kSymMinDofs) {
+            const size_t nt = (size_t)((s->nC + kSymT - 1) / kSymT);
+            s->symPart = s->dalloc<double>(nt * (nt + 1) / 2 * 2 * kSymT * s->kMax);
+            if (!s->symPart) return fail("out of device memory");
+        }
         if (!s->eleCompactC || !s->nodeCompactC || !s->Ac || !s->Ainv || !s->Wc || !s->Dc || !s->cr) return fail("out of device memory");
         cudaMemcpy(s->eleCompactC, ec.data(), sizeof(int32_t) * lc.g.cs, cudaMemcpyHostToDevice);
         cudaMemcpy(s->nodeCompactC, nc.data(), sizeof(int32_t) * lc.g.cs, cudaMemcpyHostToDevice);
@@ -1318,6 +1426,10 @@ extern "C" int top_solver_set_coarse_persistent(top_solver *s, int on)
     if (!s || on < 0 || on > 2) return TOP_ERR_ARGS;
     s->coarsePersistent = on;
     ++s->opGen;                      // captured PCG graphs change
+    if (s->assembled && s->symPart && coarse_persistent_level(s) > 0) {   // it reads A^-1 whole
+        whole_inverse(s, s->st);
+        CKL();
+    }
     return TOP_OK;
 }
 
@@ -1523,6 +1635,13 @@ int build_tail(top_solver *s, cudaStream_t st)
     return TOP_OK;
 }
 
+void whole_inverse(top_solver *s, cudaStream_t st)
+{
+    const int64_t n = s->nC;
+    dgemm(st, true, true, s->Ainv, n, s->Wc, n, s->Wc, n, n, n, n, false, true, true);
+    TOPGPU_COUNT_LAUNCH();
+}
+
 int coarsest_inverse(top_solver *s, cudaStream_t st)
 {
     const int64_t n = s->nC, nblk = (n + kDb - 1) / kDb;
@@ -1569,8 +1688,14 @@ int coarsest_inverse(top_solver *s, cudaStream_t st)
             TOPGPU_COUNT_LAUNCH();
         }
     }
-    dgemm(st, true, true, s->Ainv, n, s->Wc, n, s->Wc, n, n, n, n, false, true, true);         // W^T W
-    TOPGPU_COUNT_LAUNCH();
+    // W^T W: whole, or as packed tiles over the factor, which is no longer needed.
+    // The persistent coarse V-cycle (an option) reads it whole.
+    const unsigned nt = (unsigned)((n + kTileB - 1) / kTileB);
+    if (s->symPart) {
+        wtw_packed_kernel<<<dim3(nt, nt), kTileThreads, 0, st>>>(s->Ac, s->Wc, n);
+        TOPGPU_COUNT_LAUNCH();
+    }
+    if (!s->symPart || coarse_persistent_level(s) > 0) whole_inverse(s, st);
     return TOP_OK;
 }
 

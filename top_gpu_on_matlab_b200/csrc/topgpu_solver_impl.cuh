@@ -122,6 +122,7 @@ struct top_solver {
     double *scal = nullptr;          // device scalars for standalone reductions
     int *zeroDone = nullptr;
     int64_t nC = 0; double *Ac = nullptr, *Ainv = nullptr, *Wc = nullptr, *cr = nullptr;
+    double *symPart = nullptr;       // partial vectors of the packed symmetric coarsest product (null: A^-1 whole)
     double *Dc = nullptr;            // inverses of the coarsest factor's 32 x 32 diagonal blocks
     int32_t *eleCompactC = nullptr, *nodeCompactC = nullptr;
     bool assembled = false;
