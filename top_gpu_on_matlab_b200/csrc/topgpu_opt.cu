@@ -33,7 +33,7 @@ struct FilterState {
     KeParam<double> KEF{};   // 8x8 in k[0..63], col-major
     double *act = nullptr;   // element activity on the level-0 element slots (1/0)
     double *invD = nullptr;  // Jacobi of the filter operator, node grid
-    double *rhs = nullptr, *x = nullptr, *r = nullptr, *z = nullptr, *p = nullptr, *v = nullptr, *eg = nullptr;
+    double *x = nullptr, *r = nullptr, *z = nullptr, *p = nullptr, *v = nullptr, *eg = nullptr;
     PcgState *st = nullptr;
     double *part2 = nullptr;           // per-CTA partials of rho = z.r (the update's second sum)
     cudaGraphExec_t chunk = nullptr;   // kChunk filter-PCG iterations as one graph (built on first use)
@@ -137,33 +137,88 @@ __global__ void filter_diag_kernel(const KeParam<double> K, const double *__rest
     for (int i = 0; i < 8; ++i) d += act[idx - cdy(i) - g.PY * cdx(i) - (int)g.plane * cdz(i)] * K.k[9 * i];
     invD[idx] = (flags[idx] & kActive) && d != 0.0 ? 1.0 / d : 0.0;
 }
-// y = A_filter x (+ dot x.y), node-centric over the 8 incident elements
-__global__ void __launch_bounds__(kNodeThreads)
-filter_apply_kernel(const KeParam<double> K, const double *__restrict__ act, const double *__restrict__ x,
-                    double *__restrict__ y, Geom g, Reduce red, const int *__restrict__ done)
+// KEF in the Walsh basis of the voxel: invariant under the three axis
+// reflections, it is diagonal there, K = sum_s b[s] w_s w_s^T with
+// w_s(a) = (-1)^(s . corner a), s = s_y + 2 s_x + 4 s_z
+struct FilterWalsh { double b[8]; };
+FilterWalsh filter_walsh(const double *K)
+{
+    FilterWalsh W{};
+    for (int s = 0; s < 8; ++s) {
+        for (int a = 0; a < 8; ++a)
+            for (int c = 0; c < 8; ++c) W.b[s] += walsh_sign(s, a) * K[a + 8 * c] * walsh_sign(s, c);
+        W.b[s] /= 64.0;
+    }
+    return W;
+}
+// y = A_filter x (+ dot x.y).  As the level-0 stiffness product: a thread owns one
+// element column of a 16 x 16 tile and marches zLen layers, the (y, x) butterfly
+// of a node layer serves the elements below and above it, the node sums go
+// through shared memory in a fixed order (one barrier a layer).  43 FP64
+// operations and 5 loads an element layer instead of 72 multiply-adds and 35
+// loads a node; 64 registers, so latency hides behind 32 warps an SM.  96x192x96:
+// 51 -> 22 us a product (45 MB, 7 us at the copy rate; 9 us of FP64 operations
+// with the tiles' overlap); marching the node's 27 values instead took 44.
+constexpr int kFilterTile = 16, kFilterThreads = kFilterTile * kFilterTile;
+__global__ void __launch_bounds__(kFilterThreads, 4)
+filter_apply_kernel(const FilterWalsh W, const double *__restrict__ act, const double *__restrict__ x,
+                    double *__restrict__ y, Geom g, int zLen, Reduce red, const int *__restrict__ done)
 {
     if (done && *done) return;
-    const int q = blockIdx.x * kNodeThreads + threadIdx.x;
-    const int Y = q % g.PY, X = q / g.PY, Z = blockIdx.y;
-    const bool valid = Y < g.NY && X < g.NX;
-    const int idx = (int)(g.origin + Y + (int64_t)g.PY * X + g.plane * Z);
+    constexpr int TY = kFilterTile, NT = kFilterThreads;
+    __shared__ double so[2][3][NT];
+    const int tilesY = (g.NY + TY - 2) / (TY - 1);
+    const int y0 = (blockIdx.x % tilesY) * (TY - 1), x0 = (blockIdx.x / tilesY) * (TY - 1);
+    const int tid = threadIdx.x, ty = tid % TY, tx = tid / TY;
     const int PY = g.PY, PL = (int)g.plane;
-    double dot = 0.0;
-    if (valid) {
-        double s = 0.0;
+    const int ey = y0 - 1 + ty, ex = x0 - 1 + tx;
+    // columns past the last element read the guard column's nodes, activity 0
+    int m = (int)g.origin + min(ey, g.NY - 1) + PY * min(ex, g.NX - 1);
+    const bool nOut = ty >= 1 && tx >= 1 && ey < g.NY && ex < g.NX;
+    const int z0 = blockIdx.y * zLen, z1 = min(z0 + zLen, g.NZ);
+    auto butterfly = [](const double v[4], double h[4]) {
+        const double p0 = v[0] + v[1], m0 = v[0] - v[1], p1 = v[2] + v[3], m1 = v[2] - v[3];
+        h[0] = p0 + p1; h[1] = m0 + m1; h[2] = p0 - p1; h[3] = m0 - m1;
+    };
+    double hb[4], gt[4] = {0.0, 0.0, 0.0, 0.0}, pre[4];
+    auto load = [&](int at) {
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const int slot = idx - cdy(i) - PY * cdx(i) - PL * cdz(i);
-            const double a = act[slot];
-            double t = 0.0;
+        for (int k = 0; k < 4; ++k) pre[k] = x[at + (k & 1) + PY * (k >> 1)];
+    };
+    m += PL * (z0 - 1);
+    load(m);
+    butterfly(pre, hb);
+    double xc = 0.0, dot = 0.0, aNext = act[m];
+    load(m + PL);
+    for (int ez = z0 - 1; ez < z1; ++ez, m += PL) {
+        double ht[4];
+        butterfly(pre, ht);
+        const double xTop = pre[0], a = aNext;         // x at the column's own node of layer ez + 1
+        if (ez + 1 < z1) { load(m + 2 * PL); aNext = act[m + PL]; }
+        double G[4];
 #pragma unroll
-            for (int j = 0; j < 8; ++j) t = fma(K.k[i + 8 * j], x[slot + cdy(j) + PY * cdx(j) + PL * cdz(j)], t);
-            s = fma(a, t, s);
+        for (int k = 0; k < 4; ++k) {
+            const double v0 = W.b[k] * (a * (hb[k] + ht[k])), v1 = W.b[k + 4] * (a * (hb[k] - ht[k]));
+            G[k] = gt[k] + (v0 + v1);
+            gt[k] = v0 - v1;
+            hb[k] = ht[k];
         }
-        y[idx] = s;
-        dot = x[idx] * s;
+        if (ez >= z0) {                                // the first element only carries its top layer
+            double H[4];
+            butterfly(G, H);
+            double (*buf)[NT] = so[ez & 1];
+#pragma unroll
+            for (int k = 1; k < 4; ++k) buf[k - 1][tid] = H[k];
+            __syncthreads();
+            if (nOut) {
+                const double s = H[0] + buf[0][tid - 1] + buf[1][tid - TY] + buf[2][tid - TY - 1];
+                y[m] = s;
+                dot += xc * s;
+            }
+        }
+        xc = xTop;
     }
-    if (red.result) block_sum_to<kNodeThreads>(dot, red.partials, red.counter, red.result);
+    if (red.result) block_sum_to<NT>(dot, red.partials, red.counter, red.result);
 }
 // element values (compact) -> element slots
 __global__ void elem_to_slots_kernel(const double *__restrict__ src, const int32_t *__restrict__ eleGrid,
@@ -171,19 +226,6 @@ __global__ void elem_to_slots_kernel(const double *__restrict__ src, const int32
 {
     const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (e < Ne) dst[eleGrid[e]] = src[e] * scale;
-}
-// nodal rhs: sum of the (pre-scaled) values of the incident elements (TOP_GPU.m:975-996)
-__global__ void slots_to_nodes_kernel(const double *__restrict__ eg, Geom g, const uint8_t *__restrict__ flags,
-                                      double *__restrict__ rhs)
-{
-    const int q = blockIdx.x * kNodeThreads + threadIdx.x;
-    const int Y = q % g.PY, X = q / g.PY, Z = blockIdx.y;
-    if (Y >= g.NY || X >= g.NX) return;
-    const int idx = (int)(g.origin + Y + (int64_t)g.PY * X + g.plane * Z);
-    double s = 0;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) s += eg[idx - cdy(i) - g.PY * cdx(i) - (int)g.plane * cdz(i)];
-    rhs[idx] = (flags[idx] & kActive) ? s : 0.0;
 }
 // node -> element mean (TOP_GPU.m:1004-1005)
 __global__ void nodes_to_elem_kernel(const double *__restrict__ xn, const int32_t *__restrict__ eleGrid, Geom g,
@@ -197,18 +239,74 @@ __global__ void nodes_to_elem_kernel(const double *__restrict__ xn, const int32_
     for (int j = 0; j < 8; ++j) s += xn[slot + cdy(j) + g.PY * cdx(j) + (int)g.plane * cdz(j)];
     out[e] = s * (1.0 / 8.0);
 }
-// scalar PCG pieces (one component)
-__global__ void fpcg_init_kernel(const double *__restrict__ b, double *__restrict__ x, double *__restrict__ r,
-                                 double *__restrict__ z, double *__restrict__ p, const double *__restrict__ invD,
-                                 int64_t n, Reduce bb)
-{   // x = 0, r = b, z = M r, p = z; ||b||^2
-    double s1 = 0;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const double bi = b[i], zi = invD[i] * bi;
-        x[i] = 0.0; r[i] = bi; z[i] = zi; p[i] = zi;
-        s1 += bi * bi;
+// two grid-wide sums (s1 to *out1, s2 to *out2), per-CTA partials added in index
+// order by the CTA that finishes last; true in its thread 0, after the writes
+__device__ __forceinline__ bool two_sums_last(double s1, double s2, double *part1, double *part2, unsigned *counter,
+                                              double &out1, double &out2, unsigned nb, unsigned bid)
+{
+    __shared__ double red[2][8];
+    __shared__ bool last;
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    for (int o = 16; o > 0; o >>= 1) { s1 += __shfl_down_sync(0xffffffffu, s1, o); s2 += __shfl_down_sync(0xffffffffu, s2, o); }
+    if (lane == 0) { red[0][w] = s1; red[1][w] = s2; }
+    __syncthreads();
+    if (tid == 0) {
+        double a = 0, b = 0;
+        for (int k = 0; k < 8; ++k) a += red[0][k];
+        for (int k = 0; k < 8; ++k) b += red[1][k];
+        part1[bid] = a; part2[bid] = b;
+        __threadfence();
+        last = (atomicAdd(counter, 1u) == nb - 1);
     }
-    block_sum_to<256>(s1, bb.partials, bb.counter, bb.result);
+    __syncthreads();
+    if (!last) return false;
+    __threadfence();
+    double a = 0, b = 0;
+    for (unsigned k = tid; k < nb; k += 256) { a += ((volatile double *)part1)[k]; b += ((volatile double *)part2)[k]; }
+    for (int o = 16; o > 0; o >>= 1) { a += __shfl_down_sync(0xffffffffu, a, o); b += __shfl_down_sync(0xffffffffu, b, o); }
+    __syncthreads();
+    if (lane == 0) { red[0][w] = a; red[1][w] = b; }
+    __syncthreads();
+    if (tid != 0) return false;
+    out1 = out2 = 0.0;
+    for (int k = 0; k < 8; ++k) out1 += red[0][k];
+    for (int k = 0; k < 8; ++k) out2 += red[1][k];
+    *counter = 0;
+    return true;
+}
+// scalar PCG pieces (one component)
+// The start, one launch: the nodal right-hand side b = sum of the (pre-scaled)
+// values of the node's elements (TOP_GPU.m:975-996), x = 0, r = b, z = M r, p = z
+// on every node of the grid (the vectors are zero elsewhere), ||b||, z.r and
+// the solve's state
+__global__ void __launch_bounds__(256)
+fpcg_init_kernel(const double *__restrict__ eg, Geom g, const uint8_t *__restrict__ flags, double *__restrict__ x, double *__restrict__ r,
+                 double *__restrict__ z, double *__restrict__ p, const double *__restrict__ invD, PcgState *st, double tol, int maxIT,
+                 double *__restrict__ part1, double *__restrict__ part2, unsigned *counter)
+{
+    const int64_t n = (int64_t)g.PY * g.NX * g.NZ;
+    double s1 = 0, s2 = 0;
+    for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (int64_t)gridDim.x * blockDim.x) {
+        int Y, X, Z;
+        split3(k, g.PY, g.NX, Y, X, Z);
+        if (Y >= g.NY) continue;
+        const int idx = (int)(g.origin + Y + (int64_t)g.PY * X + g.plane * Z);
+        double b = 0;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) b += eg[idx - cdy(i) - g.PY * cdx(i) - (int)g.plane * cdz(i)];
+        if (!(flags[idx] & kActive)) b = 0.0;
+        const double zi = invD[idx] * b;
+        x[idx] = 0.0; r[idx] = b; z[idx] = zi; p[idx] = zi;
+        s1 += b * b;
+        s2 += zi * b;
+    }
+    double bb, zr;
+    if (two_sums_last(s1, s2, part1, part2, counter, bb, zr, gridDim.x, blockIdx.x)) {
+        st->normB = sqrt(bb);
+        st->rho = zr;
+        st->tol = tol; st->maxIT = maxIT; st->its = 0; st->status = 0;
+        st->done = st->normB == 0.0 ? 1 : 0;
+    }
 }
 // the filter-PCG check: same stopping rule as Solving_PCG (TOP_GPU.m:637-649)
 __device__ __forceinline__ void fpcg_check(PcgState *st)
@@ -222,8 +320,8 @@ __device__ __forceinline__ void fpcg_check(PcgState *st)
     st->rhoOld = st->rho;
 }
 // one filter-PCG step after v = A p: x += l p, r -= l v, z = M r, rr = r.r
-// and rho = z.r in one pass (four grid strides of loads ahead of the stores;
-// each thread adds its terms in index order); the CTA that completes both
+// and rho = z.r in one pass (pairs, two grid strides of loads ahead of the
+// stores); the CTA that completes both
 // sums runs the iteration's check (TOP_GPU.m:637-649) and then stores rho,
 // as the separate update, check and z.r launches did (same sums, same order)
 __global__ void __launch_bounds__(256)
@@ -234,59 +332,36 @@ fpcg_update_kernel(double *__restrict__ x, double *__restrict__ r, double *__res
     if (st->done) return;
     const double l = st->rho / st->pv;
     double s1 = 0, s2 = 0;
-    const int64_t S = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += 4 * S) {
-        double xo[4], po[4], ro[4], vo[4], dq[4];
+    const int64_t S = (int64_t)gridDim.x * blockDim.x, n2 = n >> 1;      // n a multiple of four, the bases 16-byte aligned
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n2; i += 2 * S) {
+        double xo[2][2], po[2][2], ro[2][2], vo[2][2], dq[2][2];
 #pragma unroll
-        for (int q = 0; q < 4; ++q)
-            if (i + q * S < n) {
-                const int64_t k = i + q * S;
-                xo[q] = x[k]; po[q] = p[k]; ro[q] = r[k]; vo[q] = v[k]; dq[q] = invD[k];
+        for (int q = 0; q < 2; ++q)
+            if (i + q * S < n2) {
+                const int64_t k = 2 * (i + q * S);
+                ld2(x + k, xo[q][0], xo[q][1]); ld2(p + k, po[q][0], po[q][1]); ld2(r + k, ro[q][0], ro[q][1]);
+                ld2(v + k, vo[q][0], vo[q][1]); ld2(invD + k, dq[q][0], dq[q][1]);
             }
 #pragma unroll
-        for (int q = 0; q < 4; ++q)
-            if (i + q * S < n) {
-                const int64_t k = i + q * S;
-                x[k] = xo[q] + l * po[q];
-                const double ri = ro[q] - l * vo[q];
-                r[k] = ri;
-                const double zi = dq[q] * ri;
-                z[k] = zi;
-                s1 += ri * ri;
-                s2 += zi * ri;
+        for (int q = 0; q < 2; ++q)
+            if (i + q * S < n2) {
+                const int64_t k = 2 * (i + q * S);
+                double ri[2], zi[2];
+#pragma unroll
+                for (int u = 0; u < 2; ++u) {
+                    xo[q][u] += l * po[q][u];
+                    ri[u] = ro[q][u] - l * vo[q][u];
+                    zi[u] = dq[q][u] * ri[u];
+                    s1 += ri[u] * ri[u];
+                    s2 += zi[u] * ri[u];
+                }
+                st2(x + k, xo[q][0], xo[q][1]);
+                st2(r + k, ri[0], ri[1]);
+                st2(z + k, zi[0], zi[1]);
             }
     }
-    // two block sums, each as block_sum_last forms it; the last CTA adds the
-    // partials of both in index order
-    __shared__ double red[2][8];
-    __shared__ bool last;
-    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-    const unsigned nb = gridDim.x, bid = blockIdx.x;
-    for (int o = 16; o > 0; o >>= 1) { s1 += __shfl_down_sync(0xffffffffu, s1, o); s2 += __shfl_down_sync(0xffffffffu, s2, o); }
-    if (lane == 0) { red[0][w] = s1; red[1][w] = s2; }
-    __syncthreads();
-    if (tid == 0) {
-        double a = 0, b = 0;
-        for (int k = 0; k < 8; ++k) a += red[0][k];
-        for (int k = 0; k < 8; ++k) b += red[1][k];
-        part1[bid] = a; part2[bid] = b;
-        __threadfence();
-        last = (atomicAdd(counter, 1u) == nb - 1);
-    }
-    __syncthreads();
-    if (!last) return;
-    __threadfence();
-    double a = 0, b = 0;
-    for (unsigned k = tid; k < nb; k += 256) { a += ((volatile double *)part1)[k]; b += ((volatile double *)part2)[k]; }
-    for (int o = 16; o > 0; o >>= 1) { a += __shfl_down_sync(0xffffffffu, a, o); b += __shfl_down_sync(0xffffffffu, b, o); }
-    __syncthreads();
-    if (lane == 0) { red[0][w] = a; red[1][w] = b; }
-    __syncthreads();
-    if (tid == 0) {
-        double ta = 0, tb = 0;
-        for (int k = 0; k < 8; ++k) ta += red[0][k];
-        for (int k = 0; k < 8; ++k) tb += red[1][k];
-        *counter = 0;
+    double ta, tb;
+    if (two_sums_last(s1, s2, part1, part2, counter, ta, tb, gridDim.x, blockIdx.x)) {
         st->rr = ta;
         // the iteration's check, then rho for the next direction (left as it
         // was once the solve has stopped)
@@ -294,33 +369,20 @@ fpcg_update_kernel(double *__restrict__ x, double *__restrict__ r, double *__res
         if (!st->done) st->rho = tb;
     }
 }
-__global__ void fpcg_zr_kernel(const double *__restrict__ z, const double *__restrict__ r, int64_t n, PcgState *st, Reduce red)
-{
-    if (st->done) return;
-    double s = 0;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) s += z[i] * r[i];
-    block_sum_to<256>(s, red.partials, red.counter, red.result);
-}
 __global__ void fpcg_p_kernel(double *__restrict__ p, const double *__restrict__ z, int64_t n, const PcgState *st)
 {
     if (st->done) return;
     const double beta = st->rho / st->rhoOld;
-    const int64_t S = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += 4 * S) {
-        double zo[4], po[4];
+    const int64_t S = (int64_t)gridDim.x * blockDim.x, n2 = n >> 1;
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n2; i += 2 * S) {
+        double zo[2][2], po[2][2];
 #pragma unroll
-        for (int q = 0; q < 4; ++q)
-            if (i + q * S < n) { zo[q] = z[i + q * S]; po[q] = p[i + q * S]; }
+        for (int q = 0; q < 2; ++q)
+            if (i + q * S < n2) { ld2(z + 2 * (i + q * S), zo[q][0], zo[q][1]); ld2(p + 2 * (i + q * S), po[q][0], po[q][1]); }
 #pragma unroll
-        for (int q = 0; q < 4; ++q)
-            if (i + q * S < n) p[i + q * S] = zo[q] + beta * po[q];
+        for (int q = 0; q < 2; ++q)
+            if (i + q * S < n2) st2(p + 2 * (i + q * S), zo[q][0] + beta * po[q][0], zo[q][1] + beta * po[q][1]);
     }
-}
-__global__ void fpcg_start_kernel(PcgState *st, double tol, int maxIT)
-{
-    st->normB = sqrt(st->normB);
-    st->tol = tol; st->maxIT = maxIT; st->its = 0; st->status = 0;
-    st->done = st->normB == 0.0 ? 1 : 0;
 }
 
 // ---- super-element density filter ---------------------------------------------
@@ -671,12 +733,12 @@ extern "C" int top_solver_filter_setup(top_solver *s, double rMin)
     const int64_t cs = l0.g.cs;
     if (!f.act) {
         f.act = s->galloc<double>(cs, 1); f.invD = s->galloc<double>(cs, 1);
-        f.rhs = s->galloc<double>(cs, 1); f.x = s->galloc<double>(cs, 1); f.r = s->galloc<double>(cs, 1);
+        f.x = s->galloc<double>(cs, 1); f.r = s->galloc<double>(cs, 1);
         f.z = s->galloc<double>(cs, 1); f.p = s->galloc<double>(cs, 1); f.v = s->galloc<double>(cs, 1);
         f.eg = s->galloc<double>(cs, 1);
         f.st = s->dalloc<PcgState>(1);
         f.part2 = s->dalloc<double>(4096);
-        if (!f.act || !f.invD || !f.rhs || !f.x || !f.r || !f.z || !f.p || !f.v || !f.eg || !f.st || !f.part2) {
+        if (!f.act || !f.invD || !f.x || !f.r || !f.z || !f.p || !f.v || !f.eg || !f.st || !f.part2) {
             set_error("top_solver_filter_setup: out of device memory"); return TOP_ERR_NOMEM;
         }
     }
@@ -698,27 +760,26 @@ static int filter_apply(top_solver *s, const double *src, double *tar, int *itsO
     FilterState &f = filt(s);
     DevLevel &l0 = s->L[0];
     const Geom &g = l0.g;
-    const int64_t cs = g.cs, ng = l0.ng;
+    const int64_t ng = l0.ng;
     cudaStream_t st = s->st;
-    // nodal rhs: each element adds src/8 to its nodes
-    CK(cudaMemsetAsync(f.eg - kMargin, 0, sizeof(double) * cs, st));
+    // each element adds src/8 to its nodes (only element slots are ever written: the rest of eg is zero)
     elem_to_slots_kernel<<<nb256(l0.Ne), 256, 0, st>>>(src, l0.eleGrid, l0.Ne, 1.0 / 8.0, f.eg);
     TOPGPU_COUNT_LAUNCH();
-    slots_to_nodes_kernel<<<dim3(g.nbx, g.NZ), kNodeThreads, 0, st>>>(f.eg, g, l0.flags, f.rhs);
-    TOPGPU_COUNT_LAUNCH();
     // PCG with the filter operator and Jacobi, tol_/10, maxIT_ (TOP_GPU.m:999-1001)
-    const int VB = vb(ng);
-    fpcg_init_kernel<<<VB, 256, 0, st>>>(f.rhs, f.x, f.r, f.z, f.p, f.invD, ng, s->red(&f.st->normB));
+    const int VB = (int)std::min<int64_t>(vb(ng / 2), 4 * (int64_t)s->numSMs);
+    const int IB = vb((int64_t)g.PY * g.NX * g.NZ);
+    fpcg_init_kernel<<<IB, 256, 0, st>>>(f.eg, g, l0.flags, f.x, f.r, f.z, f.p, f.invD, f.st, s->p.tol / 10.0, s->p.maxIT,
+                                         s->partials, f.part2, s->counter);
     TOPGPU_COUNT_LAUNCH();
-    fpcg_start_kernel<<<1, 1, 0, st>>>(f.st, s->p.tol / 10.0, s->p.maxIT);
-    TOPGPU_COUNT_LAUNCH();
-    fpcg_zr_kernel<<<VB, 256, 0, st>>>(f.z, f.r, ng, f.st, s->red(&f.st->rho));
-    TOPGPU_COUNT_LAUNCH();
+    // the product's z-segments: one wave of its four CTAs an SM where the layers allow it
+    const int tiles = walsh_tiles(g, kFilterTile, kFilterTile);
+    const int segs = std::max(1, std::min(g.NZ, 4 * s->numSMs / std::max(1, tiles))), zLen = (g.NZ + segs - 1) / segs;
+    const FilterWalsh W = filter_walsh(f.KEF.k);
     const int *done = &f.st->done;
     const int chunk = 8;
     // one filter-PCG iteration; every kernel returns at once after convergence
     auto iteration = [&](cudaStream_t q) {
-        filter_apply_kernel<<<dim3(g.nbx, g.NZ), kNodeThreads, 0, q>>>(f.KEF, f.act, f.p, f.v, g, s->red(&f.st->pv), done);
+        filter_apply_kernel<<<dim3(tiles, (g.NZ + zLen - 1) / zLen), kFilterThreads, 0, q>>>(W, f.act, f.p, f.v, g, zLen, s->red(&f.st->pv), done);
         TOPGPU_COUNT_LAUNCH();
         fpcg_update_kernel<<<VB, 256, 0, q>>>(f.x, f.r, f.z, f.p, f.v, f.invD, ng, f.st, s->partials, f.part2, s->counter);
         TOPGPU_COUNT_LAUNCH();
