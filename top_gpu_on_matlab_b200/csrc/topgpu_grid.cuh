@@ -234,6 +234,17 @@ struct StoreOut {   // y
         }
     }
 };
+template <typename T>
+struct CompactOut { // y in compact order (3 node + c); node[i]: the slot's node, 1-based, 0 none
+    T *y; const int32_t *node;
+    struct Pre { int32_t n; };
+    __host__ __device__ CompactOut(T *yb, const int32_t *nodeOf) : y(yb), node(nodeOf) {}
+    __device__ __forceinline__ CompactOut shift(int) const { return *this; }
+    __device__ __forceinline__ Pre pre(int i) const { return Pre{node[i]}; }
+    __device__ __forceinline__ void apply(int, const T yv[3], const Pre &p, double &) const
+    { if (p.n) for (int c = 0; c < 3; ++c) y[3 * (int64_t)(p.n - 1) + c] = yv[c]; }
+    __device__ __forceinline__ void operator()(int i, const T yv[3], double &dot) const { apply(i, yv, pre(i), dot); }
+};
 template <typename T, typename TU, typename TY>
 struct DotStoreOut { // y, and dot += u . y  (PCG: p . Ap)
     Comp3<TY *> y; Comp3<const TU *> u; int vs, o = 0;

@@ -49,6 +49,23 @@ __global__ void grid_to_compact_kernel(const TI *__restrict__ g, TO *__restrict_
 #pragma unroll
     for (int c = 0; c < 3; ++c) v[3 * n + c] = TO(g[c * cs + gi]);
 }
+__global__ void node_of_kernel(const int32_t *__restrict__ nodeGrid, int64_t Nn, int32_t *__restrict__ nodeOf)
+{
+    const int64_t n = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (n < Nn) nodeOf[nodeGrid[n]] = (int32_t)n + 1;
+}
+// a compact vector onto a whole level-0 grid vector (raw from its margin on), zero
+// where there is no node: one coalesced pass instead of clearing the vector
+// and scattering into it
+template <typename TI, typename TO>
+__global__ void spread_kernel(const TI *__restrict__ v, TO *__restrict__ g, const int32_t *__restrict__ nodeOf, int64_t cs)
+{
+    const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= cs) return;
+    const int64_t n = nodeOf[k];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) g[c * cs + k] = n ? TO(v[3 * (n - 1) + c]) : TO(0);
+}
 // E (compact, FP64) -> grid slots (FP64 + FP32); SIMP when x != nullptr
 __global__ void modulus_kernel(const double *__restrict__ src, int simp, double E0, double Emin, double p,
                                double *__restrict__ Ec, double *__restrict__ Eg, float *__restrict__ Eg32,
@@ -1075,6 +1092,12 @@ extern "C" int top_solver_create(const top_mesh *mesh, const top_solver_params *
         }
         cudaMemcpy(d.nodeGrid, ng.data(), sizeof(int32_t) * M.Nn, cudaMemcpyHostToDevice);
         cudaMemcpy(d.eleGrid, eg.data(), sizeof(int32_t) * M.Ne, cudaMemcpyHostToDevice);
+        if (l == 0) {
+            s->nodeOf = s->dalloc<int32_t>(cs);
+            if (!s->nodeOf) return fail("out of device memory");
+            node_of_kernel<<<nb256(M.Nn), 256>>>(d.nodeGrid, M.Nn, s->nodeOf + kMargin);
+            TOPGPU_COUNT_LAUNCH();
+        }
         d.diag = s->galloc<double>(cs, 3);
         d.invD64 = s->galloc<double>(cs, 3);
         d.invD32 = s->galloc<float>(cs, 3);
@@ -1756,6 +1779,21 @@ extern "C" int top_solver_assemble(top_solver *s)
 }
 
 // ---- standalone operators on compact vectors ------------------------------
+// compact v onto level l's grid vector g (its other slots zero)
+template <typename TO>
+static cudaError_t to_grid(top_solver *s, int l, const double *v, TO *g)
+{
+    DevLevel &d = s->L[l];
+    if (l == 0) {
+        spread_kernel<double, TO><<<(unsigned)((d.g.cs + 255) / 256), 256, 0, s->st>>>(v, g - kMargin, s->nodeOf, d.g.cs);
+    } else {
+        const cudaError_t e = cudaMemsetAsync(g - kMargin, 0, sizeof(TO) * 3 * d.g.cs, s->st);
+        if (e != cudaSuccess) return e;
+        compact_to_grid_kernel<double, TO><<<nb256(d.Nn), 256, 0, s->st>>>(v, g, d.nodeGrid, d.Nn, d.g.cs);
+    }
+    TOPGPU_COUNT_LAUNCH();
+    return cudaGetLastError();
+}
 extern "C" int top_solver_matvec(top_solver *s, int level, const double *u, double *y, int fp32)
 {
     if (!s || !u || !y || level < 0 || level >= s->nL) { set_error("top_solver_matvec: bad arguments"); return TOP_ERR_ARGS; }
@@ -1763,15 +1801,18 @@ extern "C" int top_solver_matvec(top_solver *s, int level, const double *u, doub
     if (level == s->nL - 1 && level > 0) { set_error("top_solver_matvec: the coarsest level is solved directly"); return TOP_ERR_ARGS; }
     DevLevel &d = s->L[level];
     const Reduce none{nullptr, nullptr, nullptr};
-    CK(cudaMemsetAsync(d.x64 - kMargin, 0, sizeof(double) * 3 * d.g.cs, s->st));
-    compact_to_grid_kernel<double, double><<<nb256(d.Nn), 256, 0, s->st>>>(u, d.x64, d.nodeGrid, d.Nn, d.g.cs);
-    TOPGPU_COUNT_LAUNCH();
     if (fp32) {                      // the operand rounded to FP32 once (as the V-cycle holds it)
-        CK(cudaMemsetAsync(d.x32 - kMargin, 0, sizeof(float) * 3 * d.g.cs, s->st));
-        compact_to_grid_kernel<double, float><<<nb256(d.Nn), 256, 0, s->st>>>(u, d.x32, d.nodeGrid, d.Nn, d.g.cs);
-        TOPGPU_COUNT_LAUNCH();
+        CK(to_grid(s, level, u, d.x32));
         level_op<float>(s, level, VecIn<float, float>{d.x32, d.g.cs}, StoreOut<float, double>{d.t64, d.g.cs}, none, nullptr);
     } else {
+        CK(to_grid(s, level, u, d.x64));
+        if (level == 0) {            // straight to compact order: no grid vector written and read back (17 us on 96x192x96)
+            l0_op<double>(s, VecIn<double, double>{d.x64, d.g.cs}, CompactOut<double>{y, s->nodeOf + kMargin}, none, nullptr);
+            CKL();
+            if (s->super) return op_err_status(s);
+            CK(cudaStreamSynchronize(s->st));          // a voxel level 0 has no bounded waits to report
+            return TOP_OK;
+        }
         level_op<double>(s, level, VecIn<double, double>{d.x64, d.g.cs}, StoreOut<double, double>{d.t64, d.g.cs}, none, nullptr);
     }
     grid_to_compact_kernel<double, double><<<nb256(d.Nn), 256, 0, s->st>>>(d.t64, y, d.nodeGrid, d.Nn, d.g.cs);
@@ -1785,9 +1826,7 @@ extern "C" int top_solver_vcycle(top_solver *s, const double *r, double *z)
     if (!s || !r || !z) return TOP_ERR_ARGS;
     if (!s->assembled) { set_error("top_solver_vcycle: assemble first"); return TOP_ERR_STATE; }
     DevLevel &l0 = s->L[0];
-    CK(cudaMemsetAsync(s->tmp - kMargin, 0, sizeof(double) * 3 * l0.g.cs, s->st));
-    compact_to_grid_kernel<double, double><<<nb256(l0.Nn), 256, 0, s->st>>>(r, s->tmp, l0.nodeGrid, l0.Nn, l0.g.cs);
-    TOPGPU_COUNT_LAUNCH();
+    CK(to_grid(s, 0, r, s->tmp));
     precond(s, s->tmp, s->z, nullptr, s->zeroDone);
     grid_to_compact_kernel<double, double><<<nb256(l0.Nn), 256, 0, s->st>>>(s->z, z, l0.nodeGrid, l0.Nn, l0.g.cs);
     TOPGPU_COUNT_LAUNCH();
@@ -1799,9 +1838,7 @@ extern "C" int top_solver_restrict(top_solver *s, int ii, const double *rF, doub
 {
     if (!s || ii < 1 || ii >= s->nL) return TOP_ERR_ARGS;
     DevLevel &f = s->L[ii - 1], &c = s->L[ii];
-    CK(cudaMemsetAsync(f.x64 - kMargin, 0, sizeof(double) * 3 * f.g.cs, s->st));
-    compact_to_grid_kernel<double, double><<<nb256(f.Nn), 256, 0, s->st>>>(rF, f.x64, f.nodeGrid, f.Nn, f.g.cs);
-    TOPGPU_COUNT_LAUNCH();
+    CK(to_grid(s, ii - 1, rF, f.x64));
     restrict_op<double>(s, ii - 1, f.x64, c.t64, nullptr);
     grid_to_compact_kernel<double, double><<<nb256(c.Nn), 256, 0, s->st>>>(c.t64, rC, c.nodeGrid, c.Nn, c.g.cs);
     TOPGPU_COUNT_LAUNCH();
@@ -1814,9 +1851,7 @@ extern "C" int top_solver_interpolate(top_solver *s, int ii, const double *xC, d
 {
     if (!s || ii < 1 || ii >= s->nL) return TOP_ERR_ARGS;
     DevLevel &f = s->L[ii - 1], &c = s->L[ii];
-    CK(cudaMemsetAsync(c.x64 - kMargin, 0, sizeof(double) * 3 * c.g.cs, s->st));
-    compact_to_grid_kernel<double, double><<<nb256(c.Nn), 256, 0, s->st>>>(xC, c.x64, c.nodeGrid, c.Nn, c.g.cs);
-    TOPGPU_COUNT_LAUNCH();
+    CK(to_grid(s, ii, xC, c.x64));
     if (c.span == 4)
         prolong_kernel<double, 4, double><<<node_grid(f.g), kNodeThreads, 0, s->st>>>(c.x64, c.g, f.t64, f.g, f.flags, nullptr, nullptr, 0.0, nullptr);
     else
@@ -2041,11 +2076,8 @@ static int pcg_run(top_solver *s, const double *bGrid, double *U, int warm, int 
 {
     DevLevel &l0 = s->L[0];
     const int64_t cs = l0.g.cs;
-    CK(cudaMemsetAsync(s->x - kMargin, 0, sizeof(double) * 3 * cs, s->st));
-    if (warm) {
-        compact_to_grid_kernel<double, double><<<nb256(l0.Nn), 256, 0, s->st>>>(U, s->x, l0.nodeGrid, l0.Nn, cs);
-        TOPGPU_COUNT_LAUNCH();
-    }
+    if (warm) CK(to_grid(s, 0, U, s->x));
+    else CK(cudaMemsetAsync(s->x - kMargin, 0, sizeof(double) * 3 * cs, s->st));
     const int rc = pcg_grid(s, bGrid, s->x, 1, itsOut, resOut);
     if (rc != TOP_OK && rc != TOP_ERR_NOT_CONVERGED) return rc;
     grid_to_compact_kernel<double, double><<<nb256(l0.Nn), 256, 0, s->st>>>(s->x, U, l0.nodeGrid, l0.Nn, cs);
@@ -2067,12 +2099,10 @@ extern "C" int top_solver_pcg_all(top_solver *s, double *U, int warm, int *its, 
     DevLevel &l0 = s->L[0];
     const int64_t cs = l0.g.cs, nd = 3 * l0.Nn;
     const int K = s->nLoads;
-    CK(cudaMemsetAsync(s->x - kMargin, 0, sizeof(double) * 3 * cs * K, s->st));
     if (warm)
-        for (int k = 0; k < K; ++k) {
-            compact_to_grid_kernel<double, double><<<nb256(l0.Nn), 256, 0, s->st>>>(U + k * nd, s->x + k * 3 * cs, l0.nodeGrid, l0.Nn, cs);
-            TOPGPU_COUNT_LAUNCH();
-        }
+        for (int k = 0; k < K; ++k) CK(to_grid(s, 0, U + k * nd, s->x + k * 3 * cs));
+    else
+        CK(cudaMemsetAsync(s->x - kMargin, 0, sizeof(double) * 3 * cs * K, s->st));
     const int rc = pcg_block(s, s->b, s->x, K, 1, its, relres);
     if (rc != TOP_OK && rc != TOP_ERR_NOT_CONVERGED) return rc;
     for (int k = 0; k < K; ++k) {
@@ -2088,10 +2118,7 @@ extern "C" int top_solver_pcg_rhs(top_solver *s, const double *b, double *U, int
 {
     if (!s || !b || !U) return TOP_ERR_ARGS;
     DevLevel &l0 = s->L[0];
-    CK(cudaMemsetAsync(s->tmp - kMargin, 0, sizeof(double) * 3 * l0.g.cs, s->st));
-    compact_to_grid_kernel<double, double><<<nb256(l0.Nn), 256, 0, s->st>>>(b, s->tmp, l0.nodeGrid, l0.Nn, l0.g.cs);
-    TOPGPU_COUNT_LAUNCH();
-    CKL();
+    CK(to_grid(s, 0, b, s->tmp));
     return pcg_run(s, s->tmp, U, warm, its, relres);
 }
 
@@ -2104,9 +2131,7 @@ extern "C" int top_solver_unit_compliance(top_solver *s, const double *U, double
     double *Ug = s->b;   // overwritten below, so re-upload afterwards would be needed: use tmp for 1 load
     if (s->nLoads != 1) { set_error("top_solver_unit_compliance: multiple load cases not supported in this call"); return TOP_ERR_ARGS; }
     Ug = s->tmp;
-    CK(cudaMemsetAsync(Ug - kMargin, 0, sizeof(double) * 3 * cs, s->st));
-    compact_to_grid_kernel<double, double><<<nb256(l0.Nn), 256, 0, s->st>>>(U, Ug, l0.nodeGrid, l0.Nn, cs);
-    TOPGPU_COUNT_LAUNCH();
+    CK(to_grid(s, 0, U, Ug));
     if (s->super)
         compliance_kmat_kernel<<<nb256(l0.Ne), 256, 0, s->st>>>(l0.KsC, Ug, 3 * cs, 1, s->weights, l0.eleGrid, l0.Ne, l0.g, ce);
     else

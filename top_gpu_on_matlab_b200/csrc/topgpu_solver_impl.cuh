@@ -77,6 +77,7 @@ struct top_solver {
         int kind = 0, ty = 16, tx = 16, ctas = 0; uint8_t *mask = nullptr;
         int2 *rng = nullptr;         // kind 3: each tile's range of layers with active nodes (null: all of them)
     };
+    int32_t *nodeOf = nullptr;       // level-0 grid slot -> compact node, 1-based (0: none), from the array's margin on
     // chunks of the level-0 vectors that the PCG vector kernels visit (ChunkList; null: all of them)
     int32_t *chunks = nullptr; int nChunks = 0;
     int numSMs = 148;

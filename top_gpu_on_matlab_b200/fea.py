@@ -173,25 +173,25 @@ class Solver:
     def matvec(self, level, u, fp32=False):
         n = 3 * self.levels[level]["numNodes"]
         u = self._dev(u, n)
-        y = torch.zeros(n, dtype=torch.float64, device="cuda")
+        y = torch.empty(n, dtype=torch.float64, device="cuda")
         check(lib().top_solver_matvec(self._h, level, u.data_ptr(), y.data_ptr(), int(fp32)), "top_solver_matvec")
         return y
 
     def vcycle(self, r):
         r = self._dev(r, self.numDOFs)
-        z = torch.zeros_like(r)
+        z = torch.empty_like(r)
         check(lib().top_solver_vcycle(self._h, r.data_ptr(), z.data_ptr()), "top_solver_vcycle")
         return z
 
     def restrict(self, ii, r):
         r = self._dev(r, 3 * self.levels[ii - 1]["numNodes"])
-        out = torch.zeros(3 * self.levels[ii]["numNodes"], dtype=torch.float64, device="cuda")
+        out = torch.empty(3 * self.levels[ii]["numNodes"], dtype=torch.float64, device="cuda")
         check(lib().top_solver_restrict(self._h, ii, r.data_ptr(), out.data_ptr()), "top_solver_restrict")
         return out
 
     def interpolate(self, ii, x):
         x = self._dev(x, 3 * self.levels[ii]["numNodes"])
-        out = torch.zeros(3 * self.levels[ii - 1]["numNodes"], dtype=torch.float64, device="cuda")
+        out = torch.empty(3 * self.levels[ii - 1]["numNodes"], dtype=torch.float64, device="cuda")
         check(lib().top_solver_interpolate(self._h, ii, x.data_ptr(), out.data_ptr()), "top_solver_interpolate")
         return out
 
@@ -245,7 +245,7 @@ class Solver:
 
     def unit_compliance(self, U):
         U = self._dev(U, self.numDOFs)
-        ce = torch.zeros(self.levels[0]["numElements"], dtype=torch.float64, device="cuda")
+        ce = torch.empty(self.levels[0]["numElements"], dtype=torch.float64, device="cuda")
         check(lib().top_solver_unit_compliance(self._h, U.data_ptr(), ce.data_ptr()), "top_solver_unit_compliance")
         return ce
 
