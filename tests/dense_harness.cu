@@ -1,11 +1,14 @@
 // Runs the coarsest level's dense kernels (topgpu_dense.cuh) on symmetric
 // diagonally dominant matrices of the sizes given and prints, per size, the
 // largest entry of A A^-1 - I, the largest difference between A^-1 and its
-// transpose, and the status flag.
+// transpose, and the status flag.  sms=N among the arguments sets the number of SMs
+// that the panel's rule reckons with for the sizes after it, neg=R makes the
+// diagonal entry of row R negative.
 #include <cstdio>
 #include <cstdlib>
 #include <algorithm>
 #include <cmath>
+#include <cstring>
 #include <vector>
 #include "topgpu_dense.cuh"
 
@@ -14,15 +17,18 @@ using namespace topgpu;
 
 int main(int argc, char **argv)
 {
-    CK(cudaFuncSetAttribute(chol_diag_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDiagSmem));
-    CK(cudaFuncSetAttribute(chol_panel_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPanelSmem));
+    CK(chol_smem_attr());
+    int sms = 148, neg = -1;
     for (int a = 1; a < argc; ++a) {
+        if (!std::strncmp(argv[a], "sms=", 4)) { sms = std::atoi(argv[a] + 4); continue; }
+        if (!std::strncmp(argv[a], "neg=", 4)) { neg = std::atoi(argv[a] + 4); continue; }
         const int64_t n = std::atoi(argv[a]);
         std::vector<double> A((size_t)(n * n)), X(A.size());
         uint64_t h = 88172645463325252ull + n;
         auto rnd = [&] { h ^= h << 13; h ^= h >> 7; h ^= h << 17; return double(h >> 11) * 0x1p-53 - 0.5; };
         for (int64_t j = 0; j < n; ++j)      // off-diagonal row sums below 1, diagonal in [2, 3]: condition below 4
             for (int64_t i = j; i < n; ++i) A[i + n * j] = A[j + n * i] = i == j ? 2.5 + rnd() : 2.0 * rnd() / double(n);
+        if (neg >= 0 && neg < n) A[neg + n * neg] = -1.0;
         double *dA, *W, *I, *D;
         int *st;
         const size_t b = sizeof(double) * A.size();
@@ -35,9 +41,9 @@ int main(int argc, char **argv)
             const int64_t rest = n - k0 - kPb;
             if (rest <= 0) break;
             const unsigned nt = (unsigned)((rest + kTileB - 1) / kTileB);
-            chol_panel_kernel<<<nt, kPanelThreads, kPanelSmem>>>(dA, n, k0, D);
-            chol_trail_kernel<<<dim3(nt, 1), kTileThreads>>>(dA, n, k0, 0);
-            if (nt > 1) chol_trail_kernel<<<dim3(nt, nt - 1), kTileThreads>>>(dA, n, k0, 1);
+            chol_panel(dA, n, k0, D, sms, 0);
+            chol_next(dA, n, k0, 0);
+            if (nt > 2) chol_trail_kernel<<<dim3(nt, nt - 2), kTileThreads>>>(dA, n, k0, 2);
         }
         place_dinv_kernel<<<(unsigned)((n + kDb - 1) / kDb), kDb * kDb>>>(D, W, n);
         for (int64_t hs = kDb; hs < n; hs *= 2) {

@@ -6,8 +6,9 @@
 //     a time: chol_diag_kernel factors the 128 x 128 diagonal block in one
 //     CTA's shared memory (and inverts its four 32 x 32 diagonal blocks),
 //     chol_panel_kernel forms the panel below it, L21 = A21 L11^-T block by
-//     block, and chol_trail_kernel applies the four rank-32 updates
-//     A22 -= L21 L21^T to every trailing tile in one pass.  Each entry still
+//     block, and chol_next_kernel (the next step's columns) and chol_trail_kernel
+//     (the others) apply the four rank-32 updates A22 -= L21 L21^T to every
+//     trailing tile in one pass.  Each entry still
 //     receives the 32-column blocks' contributions one after another, each
 //     summed from zero, as a sweep of one block at a time gives them;
 //   * W = L^-1 by 2x2 block inversion, [L11 0; L21 L22]^-1 =
@@ -16,11 +17,13 @@
 //   * A^-1 = W^T W on the lower tiles, mirrored, skipping the zero blocks of W.
 //
 // Measured on one B200, factor and inverse (bit-identical to the sweep of one
-// 32-column block a step on SIMT tiles that this replaces): n = 336 506 -> 312
-// us, n = 1386 2.31 -> 1.23 ms, n = 4131 12.4 -> 5.8 ms (the last factor and
-// trailing updates 3.4 ms, W 1.4 ms, W^T W 0.9 ms; its 35 G multiply-adds take
-// 2.5 ms at the FP64 peak).  Small sizes are bound by the diagonal blocks' chain
-// of square roots and divisions, about 11 us a block of 32 columns.
+// 32-column block a step on SIMT tiles that this replaces): n = 336 506 -> 265
+// us, n = 1386 2.31 -> 1.07 ms, n = 4131 12.4 -> 5.35 ms (the last factor and
+// trailing updates 3.0 ms, W 1.4 ms, W^T W 0.9 ms; its 35 G multiply-adds take
+// 2.5 ms at the FP64 peak).  Small sizes are bound by the chain diagonal block ->
+// panel -> next columns, 37 + 8 + 6..8 us a step of 128 columns at n = 1386
+// (one warp a block, panels of 64 rows a CTA, 64 x 64 tiles throughout: 49 + 15
+// + 13 us), and that by the pivots' square roots and reciprocals (below).
 //
 // All products run on mma.sync.m8n8k4.f64 through one tile loop (64 x 64
 // outputs, 4 warps of 32 x 32, K steps of 16 double-buffered in shared memory)
@@ -203,79 +206,121 @@ inv_level_kernel(const double *__restrict__ L, double *__restrict__ W, double *_
 }
 
 // ---- factorisation ----------------------------------------------------------------
-// One warp factors the 32 x 32 block S (column-major, stride ld, lower part
-// read and overwritten by L) with lane r holding row r: a[i] is entry
-// (r, j + i) while column j is eliminated, so the loop body is the same for
-// every column and stays in the instruction cache (the fully unrolled form was
-// bound by instruction fetch: 42 us cold against 16.8 us repeated).  A second
-// warp follows column by column with W = L^-1, lane c solving L w = e_c, so
-// the inversion hides behind the pivots' square roots and divisions, whose
-// latency bounds the block.  status: set when a pivot is not positive (the
-// pivot is then taken as 1).  Called by 64 threads (warps 0 and 1).
+// Six warps factor the 32 x 32 block S (column-major, stride ld, lower part read
+// and overwritten by L, upper part by leftovers) and invert it.  Warp w < 4 holds
+// columns 8 w .. 8 w + 7, lane r row r, and eliminates with its columns while the
+// later ones follow; warps 4 and 5 follow with W = L^-1, solving L w = e_c, two lanes a
+// column (even and odd rows).  What
+// bounds the block is the chain pivot -> square root -> reciprocal -> column -> next
+// pivot (104 + 75 cycles for the first two, 23 a multiply-add, 27 a shuffle).  So
+// the lane of the next row forms its pivot from its own entries before the column
+// goes to shared memory, a column's owner has at most seven updates to issue, and it
+// tells the others on the column's own mbarrier (ready[j], one phase a block; no
+// cycles lost on the chain, where a barrier they all meet at cost 70 a column).
+// a[i] is entry (r, j + i) while the owner eliminates column j, so the loop body is
+// the same for every column and stays in the instruction cache.  status: set when a
+// pivot is not positive (the pivot is then taken as 1).
 constexpr int kCholLd = kDb + 2;         // column j of L from row j + 1 on: sL[j][i] = L[j + 1 + i][j]
-__device__ __forceinline__ void chol_block_warps(double *S, int ld, double (*sL)[kCholLd], double *sInv, double *Ds, int ldd, int *status)
+constexpr int kCholWarps = 6;
+__device__ __forceinline__ void chol_ready(uint64_t *ready)
+{
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" :: "r"((unsigned)__cvta_generic_to_shared(ready)) : "memory");
+}
+// bounded: past the limit the factor is flagged and the warp goes on
+__device__ __forceinline__ void chol_await(uint64_t *ready, int phase, int *status)
+{
+    const unsigned a = (unsigned)__cvta_generic_to_shared(ready);
+    unsigned ok = 0;
+    for (int tries = 0; !ok && tries < (1 << 20); ++tries)
+        asm volatile("{.reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p;}" : "=r"(ok) : "r"(a), "r"(phase) : "memory");
+    if (!ok) atomicExch(status, 1);
+}
+__device__ __forceinline__ void chol_block_warps(int w, double *S, int ld, double (*sL)[kCholLd], double *sInv, double *Ds, int ldd, uint64_t *ready, int phase, int *status)
 {
     const int r = threadIdx.x & 31;
-    if (threadIdx.x < 32) {
-        double a[kDb];
+    if (w < 4) {
+        double a[8];
 #pragma unroll
-        for (int c = 0; c < kDb; ++c) a[c] = c <= r ? S[r + ld * c] : 0.0;
+        for (int i = 0; i < 8; ++i) a[i] = 8 * w + i <= r ? S[r + ld * (8 * w + i)] : 0.0;
 #pragma unroll 1
-        for (int j = 0; j < kDb; ++j) {
-            double d = __shfl_sync(0xffffffffu, a[0], j);
-            if (!(d > 0.0)) { if (r == j) atomicExch(status, 1); d = 1.0; }
-            const double ljj = sqrt(d), rl = 1.0 / ljj;
-            const double l = r == j ? ljj : a[0] * rl;       // rows above j hold leftovers that nothing reads
-            if (r > j) sL[j][r - j - 1] = l;
-            if (r == j) sInv[j] = rl;
-            if (r >= j) S[r + ld * j] = l;
-            asm volatile("bar.sync 1, 64;" ::: "memory");    // column j to both warps
+        for (int j = 0; j < 8 * w; ++j) {                        // earlier owners' columns
+            chol_await(ready + j, phase, status);
+            const double l = S[r + ld * j];
 #pragma unroll
-            for (int i = 1; i < kDb; i += 2) {
-                // past the block's last column: leftovers, never read back
-                const double2 lc = *reinterpret_cast<const double2 *>(&sL[j][i - 1]);
-                a[i - 1] = fma(-l, lc.x, a[i]);
-                if (i + 1 < kDb) a[i] = fma(-l, lc.y, a[i + 1]);
+            for (int i = 0; i < 8; i += 2) {
+                const double2 lc = *reinterpret_cast<const double2 *>(S + ld * j + 8 * w + i);
+                a[i] = fma(-l, lc.x, a[i]);
+                a[i + 1] = fma(-l, lc.y, a[i + 1]);
             }
         }
-    } else {
-        double w[kDb];                   // w[i] = entry (j + i, c) of W at step j
-#pragma unroll
-        for (int i = 0; i < kDb; ++i) w[i] = i == r ? 1.0 : 0.0;
+        double d = __shfl_sync(0xffffffffu, a[0], 8 * w);
+        bool bad = false;
 #pragma unroll 1
-        for (int j = 0; j < kDb; ++j) {
-            asm volatile("bar.sync 1, 64;" ::: "memory");
-            const double x = w[0] * sInv[j];
-            Ds[j + ldd * r] = x;
+        for (int j = 8 * w; j < 8 * w + 8; ++j) {
+            const bool ok = d > 0.0;                             // beside the root: a test ahead of it cost 85 cycles a column
+            const double root = sqrt(d), inv = 1.0 / root;
+            const double ljj = ok ? root : 1.0, rl = ok ? inv : 1.0;
+            bad = bad || !ok;
+            const double l = a[0] * rl;                          // rows above j hold leftovers that nothing uses
+            d = __shfl_sync(0xffffffffu, fma(-l, l, a[1]), j + 1);     // the next pivot; past the segment: not used
+            const double lj = r == j ? ljj : l;
+            sL[j][(r - j - 1) & 31] = lj;
+            sInv[j] = rl;
+            S[r + ld * j] = lj;
+            __syncwarp();
+            if (r == 0) chol_ready(ready + j);
 #pragma unroll
-            for (int i = 1; i < kDb; i += 2) {
+            for (int i = 1; i < 8; i += 2) {
+                // past the warp's last column: leftovers, never read back
                 const double2 lc = *reinterpret_cast<const double2 *>(&sL[j][i - 1]);
-                w[i - 1] = fma(-lc.x, x, w[i]);
-                if (i + 1 < kDb) w[i] = fma(-lc.y, x, w[i + 1]);
+                a[i - 1] = fma(-l, lc.x, a[i]);
+                if (i + 1 < 8) a[i] = fma(-l, lc.y, a[i + 1]);
             }
+        }
+        if (bad && r == 0) atomicExch(status, 1);
+    } else {
+        const int h = r >> 4, c = (r & 15) + 16 * (w - 4);
+        double x[kDb / 2];               // x[i] = entry (j + 2 i + h, c) of W at even steps j
+#pragma unroll
+        for (int i = 0; i < kDb / 2; ++i) x[i] = 2 * i + h == c ? 1.0 : 0.0;
+#pragma unroll 1
+        for (int j = 0; j < kDb; j += 2) {
+            chol_await(ready + j, phase, status);
+            const double y0 = __shfl_sync(0xffffffffu, x[0] * sInv[j], r & 15);
+            // row j + 2 i + h: L[row][j] = sL[j][row - j - 1] (i = 0 of the even half is row j itself: not used again)
+#pragma unroll
+            for (int i = 0; i < kDb / 2; ++i) x[i] = fma(-sL[j][i || h ? 2 * i + h - 1 : 0], y0, x[i]);
+            chol_await(ready + j + 1, phase, status);
+            const double y1 = __shfl_sync(0xffffffffu, x[0] * sInv[j + 1], (r & 15) + 16);
+            Ds[j + h + ldd * c] = h ? y1 : y0;
+            // row j + 2 i + h of the next pair, i from 1: sL[j + 1][row - j - 2]
+#pragma unroll
+            for (int i = 1; i < kDb / 2; ++i) x[i - 1] = fma(-sL[j + 1][2 * i + h - 2], y1, x[i]);
         }
     }
 }
-// 8 x 32 outputs by one warp from shared memory: acc[J] += sum_{k < 32}
+// 8 x 8 NJ outputs by one warp from shared memory: acc[J] = sum_{k < 32}
 // a(row g, k) b(col, k), a at Ap[row + lda k], b at Bp[col + ldb k]
-__device__ __forceinline__ void dmma_8x32(const double *Ap, int lda, const double *Bp, int ldb, double (&acc)[4][2])
+template <int NJ>
+__device__ __forceinline__ void dmma_8x(const double *Ap, int lda, const double *Bp, int ldb, double (&acc)[NJ][2])
 {
     const int lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
 #pragma unroll
-    for (int J = 0; J < 4; ++J) acc[J][0] = acc[J][1] = 0.0;
+    for (int J = 0; J < NJ; ++J) acc[J][0] = acc[J][1] = 0.0;
 #pragma unroll
     for (int kk = 0; kk < kDb; kk += 4) {
         const double a = Ap[g + lda * (kk + q)];
 #pragma unroll
-        for (int J = 0; J < 4; ++J) dmma_8x8x4(acc[J][0], acc[J][1], a, Bp[8 * J + g + ldb * (kk + q)]);
+        for (int J = 0; J < NJ; ++J) dmma_8x8x4(acc[J][0], acc[J][1], a, Bp[8 * J + g + ldb * (kk + q)]);
     }
 }
-// the warp's 8 x 32 outputs into column-major Sp (stride ld): assigned, or subtracted
-__device__ __forceinline__ void put_8x32(double *Sp, int ld, const double (&acc)[4][2], bool subtract)
+// the warp's 8 x 8 NJ outputs into column-major Sp (stride ld): assigned, or subtracted
+template <int NJ>
+__device__ __forceinline__ void put_8x(double *Sp, int ld, const double (&acc)[NJ][2], bool subtract)
 {
     const int lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
 #pragma unroll
-    for (int J = 0; J < 4; ++J)
+    for (int J = 0; J < NJ; ++J)
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             double *p = Sp + g + ld * (8 * J + 2 * q + h);
@@ -283,70 +328,114 @@ __device__ __forceinline__ void put_8x32(double *Sp, int ld, const double (&acc)
         }
 }
 
-constexpr int kDiagLd = kPb + 4, kDiagThreads = 256;
-constexpr size_t kDiagSmem = sizeof(double) * (kPb * kDiagLd + kDb * kCholLd + kDb + kDb * 36);
-// The 128 x 128 diagonal block at column k0 in one CTA: L over A's lower part,
+constexpr int kDiagLd = kPb + 4, kDiagThreads = 512;
+constexpr size_t kDiagSmem = sizeof(double) * (kPb * kDiagLd + kDb * kCholLd + kDb + 2 * kDb * 36) + sizeof(uint64_t) * kDb;
+// The 128 x 128 diagonal block at column k0 in one CTA, 37 us: four 32-column blocks of
+// about 11,700 cycles (their chain), the products between them 18,000 cycles at
+// one SM's FP64 rate.  L over A's lower part,
 // the 32 x 32 diagonal blocks' inverses to Dinv (rows / columns past n the identity).
+// Between two 32-column blocks only the next diagonal block is brought up to
+// date; the other updates are the remaining warps' while five factor it.
 __global__ void __launch_bounds__(kDiagThreads)
 chol_diag_kernel(double *A, int64_t n, int64_t k0, double *Dinv, int *status)
 {
     extern __shared__ __align__(16) double dsm[];
     double *S = dsm;                                                     // [128 columns][132]
     double (*sL)[kCholLd] = reinterpret_cast<double (*)[kCholLd]>(dsm + kPb * kDiagLd);
-    double *sInv = dsm + kPb * kDiagLd + kDb * kCholLd, *Ds = sInv + kDb;    // Ds: [32 columns][36]
+    double *sInv = dsm + kPb * kDiagLd + kDb * kCholLd, *DsAll = sInv + kDb;    // two of [32 columns][36]
+    uint64_t *ready = reinterpret_cast<uint64_t *>(DsAll + 2 * kDb * 36);
     const int t = threadIdx.x, warp = t >> 5;
+    constexpr int rest = kDiagThreads / 32 - kCholWarps;                 // warps beside the factorising ones
+    const int idle = warp - kCholWarps;                                  // their index among those
     const int wb = n - k0 < kPb ? (int)(n - k0) : kPb, nb = (wb + kDb - 1) / kDb;
+    if (t < kDb) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"((unsigned)__cvta_generic_to_shared(ready + t)) : "memory");
+    if (wb == kPb) {                     // the whole square, sixteen loads in flight; its upper part is cleared here
+        const double *a = A + k0 + (t & (kPb - 1)) + n * (k0 + t / kPb);
+        const int i = t & (kPb - 1);
 #pragma unroll 16
-    for (int u = 0; u < kPb * kPb / kDiagThreads; ++u) {                 // 16 loads in flight
-        const int e = t + u * kDiagThreads, i = e % kPb, c = e / kPb;
-        S[i + kDiagLd * c] = (i < wb && c <= i) ? A[(k0 + i) + n * (k0 + c)] : (i == c ? 1.0 : 0.0);
+        for (int u = 0; u < kPb * kPb / kDiagThreads; ++u) {
+            const int c = t / kPb + u * (kDiagThreads / kPb);
+            const double v = a[n * (u * (kDiagThreads / kPb))];
+            S[i + kDiagLd * c] = c <= i ? v : 0.0;
+        }
+    } else {
+        for (int e = t; e < kPb * kPb; e += kDiagThreads) {
+            const int i = e % kPb, c = e / kPb;
+            S[i + kDiagLd * c] = (i < wb && c <= i) ? A[(k0 + i) + n * (k0 + c)] : (i == c ? 1.0 : 0.0);
+        }
     }
     __syncthreads();
+    auto put_columns = [&](int b, int t0, int step) {                    // block b's columns of L
+        const int h = kPb - kDb * b;
+        for (int e = t0; e < kDb * h; e += step) {
+            const int c = kDb * b + e / h, i = kDb * b + e % h;
+            if (i < wb && c <= i) A[(k0 + i) + n * (k0 + c)] = S[i + kDiagLd * c];
+        }
+    };
     for (int b = 0; b < nb; ++b) {
-        const int c0 = kDb * b;
-        if (t < 64) chol_block_warps(S + c0 + kDiagLd * c0, kDiagLd, sL, sInv, Ds, 36, status);
-        __syncthreads();
-        for (int e = t; e < kDb * kDb; e += kDiagThreads) Dinv[(k0 / kDb + b) * kDb * kDb + e] = Ds[e % kDb + 36 * (e / kDb)];
-        // rows below the block: L = A D^T, eight rows a warp at a time
-        for (int r = c0 + kDb + 8 * warp; r < kDb * nb; r += kDiagThreads / 4) {
-            double acc[4][2];
-            dmma_8x32(S + r + kDiagLd * c0, kDiagLd, Ds, 36, acc);
-            __syncwarp();
-            put_8x32(S + r + kDiagLd * c0, kDiagLd, acc, false);
+        const int c0 = kDb * b, p0 = c0 - kDb;
+        double *Ds = DsAll + (b & 1) * kDb * 36;
+        if (warp < kCholWarps) {
+            if (b) {                     // the block's own update by the last block's columns
+                if (warp < 4) {
+                    double acc[4][2];
+                    const int r = c0 + 8 * warp;
+                    dmma_8x(S + r + kDiagLd * p0, kDiagLd, S + c0 + kDiagLd * p0, kDiagLd, acc);
+                    put_8x(S + r + kDiagLd * c0, kDiagLd, acc, true);
+                }
+                asm volatile("bar.sync 1, %0;" :: "n"(32 * kCholWarps) : "memory");
+            }
+            chol_block_warps(warp, S + c0 + kDiagLd * c0, kDiagLd, sL, sInv, Ds, 36, ready, b & 1, status);
+        } else if (b) {
+            // the other entries' update by the last block's columns, and its inverse
+            int item = 0;
+            for (int b2 = b; b2 < nb; ++b2)
+                for (int r = kDb * b2 + (b2 == b ? kDb : 0); r < kDb * nb; r += 8) {
+                    if (item++ % rest != idle) continue;
+                    double acc[4][2];
+                    dmma_8x(S + r + kDiagLd * p0, kDiagLd, S + kDb * b2 + kDiagLd * p0, kDiagLd, acc);
+                    put_8x(S + r + kDiagLd * kDb * b2, kDiagLd, acc, true);
+                }
+            const double *Dp = DsAll + ((b - 1) & 1) * kDb * 36;
+            const int ti = 32 * idle + (t & 31);
+            put_columns(b - 1, ti, 32 * rest);
+            for (int e = ti; e < kDb * kDb; e += 32 * rest) Dinv[(k0 / kDb + b - 1) * kDb * kDb + e] = Dp[e % kDb + 36 * (e / kDb)];
         }
         __syncthreads();
-        // the later columns' rank-32 update
-        for (int b2 = b + 1; b2 < nb; ++b2)
-            for (int r = kDb * b2 + 8 * warp; r < kDb * nb; r += kDiagThreads / 4) {
-                double acc[4][2];
-                dmma_8x32(S + r + kDiagLd * c0, kDiagLd, S + kDb * b2 + kDiagLd * c0, kDiagLd, acc);
-                put_8x32(S + r + kDiagLd * kDb * b2, kDiagLd, acc, true);
-            }
+        // rows below the block: L = A D^T, eight rows a warp
+        for (int r = c0 + kDb + 8 * warp; r < kDb * nb; r += kDiagThreads / 4) {
+            double acc[4][2];
+            dmma_8x(S + r + kDiagLd * c0, kDiagLd, Ds, 36, acc);
+            __syncwarp();
+            put_8x(S + r + kDiagLd * c0, kDiagLd, acc, false);
+        }
         __syncthreads();
     }
-    for (int e = t; e < kPb * kPb; e += kDiagThreads) {
-        const int i = e % kPb, c = e / kPb;
-        if (i < wb && c <= i) A[(k0 + i) + n * (k0 + c)] = S[i + kDiagLd * c];
-    }
+    for (int e = t; e < kDb * kDb; e += kDiagThreads)
+        Dinv[(k0 / kDb + nb - 1) * kDb * kDb + e] = DsAll[((nb - 1) & 1) * kDb * 36 + e % kDb + 36 * (e / kDb)];
+    put_columns(nb - 1, t, kDiagThreads);
 }
-// The panel below a full 128-column diagonal block: 64 rows a CTA in shared
+// The panel below a full 128-column diagonal block: R rows a CTA in shared
 // memory, block by block L_b = A_b D_b^T and A_b2 -= L_b L11(b2, b)^T for the
-// blocks b2 to its right.
-constexpr int kPanelLd = kTileB + 4;
-constexpr size_t kPanelSmem = sizeof(double) * (kPb * kPanelLd + 10 * kDb * 36);
+// blocks b2 to its right.  Eight warps, each eight rows by R / 2 columns of a
+// block: the fewer rows a CTA has, the shorter its chain of ten products, which is
+// what a panel that leaves the chip idle waits for (the products' rate on one SM).
 constexpr int kPanelThreads = 256;
+template <int R> constexpr size_t kPanelSmem = sizeof(double) * (kPb * (R + 4) + 10 * kDb * 36);
+template <int R>
 __global__ void __launch_bounds__(kPanelThreads)
 chol_panel_kernel(double *A, int64_t n, int64_t k0, const double *__restrict__ Dinv)
 {
+    constexpr int ld = R + 4, J = R / 16;                // J 8-column tiles a warp
     extern __shared__ __align__(16) double psm[];
-    double *S = psm, *Bl = psm + kPb * kPanelLd;         // Bl: D_0..D_3, then L11(b2, b) for b < b2
+    double *S = psm, *Bl = psm + kPb * ld;               // Bl: D_0..D_3, then L11(b2, b) for b < b2
     const int t = threadIdx.x, warp = t >> 5;
-    const int64_t i0 = k0 + kPb + (int64_t)blockIdx.x * kTileB;
-    const bool full = i0 + kTileB <= n;
+    const int64_t i0 = k0 + kPb + (int64_t)blockIdx.x * R;
+    const bool full = i0 + R <= n;
 #pragma unroll 16
-    for (int u = 0; u < kTileB * kPb / kPanelThreads; ++u) {             // 16 loads in flight
-        const int e = t + u * kPanelThreads, i = e % kTileB, c = e / kTileB;
-        S[i + kPanelLd * c] = full || i0 + i < n ? A[(i0 + i) + n * (k0 + c)] : 0.0;
+    for (int u = 0; u < R * kPb / kPanelThreads; ++u) {                  // 16 loads in flight
+        const int e = t + u * kPanelThreads, i = e % R, c = e / R;
+        S[i + ld * c] = full || i0 + i < n ? A[(i0 + i) + n * (k0 + c)] : 0.0;
     }
 #pragma unroll
     for (int b = 0; b < 4; ++b)
@@ -365,25 +454,37 @@ chol_panel_kernel(double *A, int64_t n, int64_t k0, const double *__restrict__ D
                 Bl[(4 + b2 * (b2 - 1) / 2 + b) * kDb * 36 + e % kDb + 36 * (e / kDb)] = A[(k0 + kDb * b2 + e % kDb) + n * (k0 + kDb * b + e / kDb)];
             }
     __syncthreads();
-    // a warp's eight rows are its own from here on: no CTA-wide barrier
-    double *R = S + 8 * warp;
+    // with all 32 columns a warp's eight rows are its own from here on: no CTA-wide barrier
+    auto meet = [] { if (J == 4) __syncwarp(); else __syncthreads(); };
+    double *Rw = S + 8 * (warp % (R / 8));
+    const int cw = (warp / (R / 8)) * (8 * J);           // the warp's first column in a block
     for (int b = 0; b < 4; ++b) {
-        double acc[4][2];
-        dmma_8x32(R + kPanelLd * kDb * b, kPanelLd, Bl + b * kDb * 36, 36, acc);
-        __syncwarp();
-        put_8x32(R + kPanelLd * kDb * b, kPanelLd, acc, false);
-        __syncwarp();
+        double acc[J][2];
+        dmma_8x(Rw + ld * kDb * b, ld, Bl + b * kDb * 36 + cw, 36, acc);
+        meet();
+        put_8x(Rw + ld * (kDb * b + cw), ld, acc, false);
+        meet();
         for (int b2 = b + 1; b2 < 4; ++b2) {
-            dmma_8x32(R + kPanelLd * kDb * b, kPanelLd, Bl + (4 + b2 * (b2 - 1) / 2 + b) * kDb * 36, 36, acc);
-            put_8x32(R + kPanelLd * kDb * b2, kPanelLd, acc, true);
+            dmma_8x(Rw + ld * kDb * b, ld, Bl + (4 + b2 * (b2 - 1) / 2 + b) * kDb * 36 + cw, 36, acc);
+            put_8x(Rw + ld * (kDb * b2 + cw), ld, acc, true);
         }
-        __syncwarp();
+        meet();
     }
     __syncthreads();
-    for (int e = t; e < kTileB * kPb; e += kPanelThreads) {
-        const int i = e % kTileB, c = e / kTileB;
-        if (i0 + i < n) A[(i0 + i) + n * (k0 + c)] = S[i + kPanelLd * c];
+    for (int e = t; e < R * kPb; e += kPanelThreads) {
+        const int i = e % R, c = e / R;
+        if (i0 + i < n) A[(i0 + i) + n * (k0 + c)] = S[i + ld * c];
     }
+}
+// Its launch for the rows below column k0 + 128 on st: the fewest rows a CTA that
+// still make one wave of the SMs.
+inline void chol_panel(double *A, int64_t n, int64_t k0, const double *Dinv, int sms, cudaStream_t st)
+{
+    const int64_t rest = n - k0 - kPb;
+    auto ctas = [&](int R) { return (unsigned)((rest + R - 1) / R); };
+    if (ctas(16) <= (unsigned)sms) chol_panel_kernel<16><<<ctas(16), kPanelThreads, kPanelSmem<16>, st>>>(A, n, k0, Dinv);
+    else if (ctas(32) <= (unsigned)sms) chol_panel_kernel<32><<<ctas(32), kPanelThreads, kPanelSmem<32>, st>>>(A, n, k0, Dinv);
+    else chol_panel_kernel<64><<<ctas(64), kPanelThreads, kPanelSmem<64>, st>>>(A, n, k0, Dinv);
 }
 // A22 -= L21 L21^T on the lower tiles of the trailing matrix (first row and
 // column k0 + 128) from tile column jt on, the step's four blocks one after
@@ -413,6 +514,77 @@ chol_trail_kernel(double *A, int64_t n, int64_t k0, int jt)
                 for (int h = 0; h < 2; ++h) { c[I][J][h] -= acc[I][J][h]; acc[I][J][h] = 0.0; }
     });
     each_out(c, [&](int r, int col, double &v) { const int i = i0 + r, j = j0 + col; if (i < m && j < m) C[i + n * j] = v; });
+}
+
+// The same update of the next step's 128 columns alone, ahead of the others: what the
+// next diagonal block waits for.  32 x 32 outputs a CTA with both operands' 128
+// columns in shared memory at once: a short chain on many SMs, where the 64 x 64
+// tiles of the kernel above take four times the products an SM.
+constexpr int kNextThreads = 256, kNextLd = kDb + 4;
+constexpr size_t kNextSmem = sizeof(double) * 2 * kPb * kNextLd;
+__global__ void __launch_bounds__(kNextThreads)
+chol_next_kernel(double *A, int64_t n, int64_t k0)
+{
+    extern __shared__ __align__(16) double nsm[];
+    double *Li = nsm, *Lj = nsm + kPb * kNextLd;
+    const int i0 = blockIdx.x * kDb, j0 = blockIdx.y * kDb;
+    if (j0 > i0) return;
+    const int t = threadIdx.x, warp = t >> 5, g = (t & 31) >> 2, q = t & 3;
+    const int64_t t0 = k0 + kPb;
+    const int m = (int)(n - t0);
+    const double *L = A + t0 + n * k0;
+    double *C = A + t0 * (1 + n);
+    const int r0 = 8 * (warp & 3), c0 = 16 * (warp >> 2);                // the warp's 8 x 16 outputs
+    double c[2][2], acc[2][2];
+#pragma unroll
+    for (int J = 0; J < 2; ++J)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int i = i0 + r0 + g, j = j0 + c0 + 8 * J + 2 * q + h;
+            c[J][h] = (i < m && j < m) ? C[i + n * j] : 0.0;
+        }
+#pragma unroll
+    for (int u = 0; u < kDb * kPb / kNextThreads; ++u) {
+        const int e = t + u * kNextThreads, r = e % kDb, k = e / kDb;
+        Li[r + kNextLd * k] = i0 + r < m ? L[i0 + r + n * k] : 0.0;
+        Lj[r + kNextLd * k] = j0 + r < m ? L[j0 + r + n * k] : 0.0;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int b = 0; b < 4; ++b) {
+        dmma_8x(Li + r0 + kNextLd * kDb * b, kNextLd, Lj + c0 + kNextLd * kDb * b, kNextLd, acc);
+#pragma unroll
+        for (int J = 0; J < 2; ++J)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) c[J][h] -= acc[J][h];
+    }
+#pragma unroll
+    for (int J = 0; J < 2; ++J)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int i = i0 + r0 + g, j = j0 + c0 + 8 * J + 2 * q + h;
+            if (i < m && j < m) C[i + n * j] = c[J][h];
+        }
+}
+inline void chol_next(double *A, int64_t n, int64_t k0, cudaStream_t st)
+{
+    const int64_t rest = n - k0 - kPb, tiles = (rest + kDb - 1) / kDb;
+    chol_next_kernel<<<dim3((unsigned)tiles, (unsigned)(tiles < 4 ? tiles : 4)), kNextThreads, kNextSmem, st>>>(A, n, k0);
+}
+
+// opts the factorisation's kernels into their shared memory
+inline cudaError_t chol_smem_attr()
+{
+    cudaError_t e = cudaSuccess;
+    auto opt = [&](auto kernel, size_t bytes) {
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    };
+    opt(chol_diag_kernel, kDiagSmem);
+    opt(chol_panel_kernel<16>, kPanelSmem<16>);
+    opt(chol_panel_kernel<32>, kPanelSmem<32>);
+    opt(chol_panel_kernel<64>, kPanelSmem<64>);
+    opt(chol_next_kernel, kNextSmem);
+    return e;
 }
 
 // copy the diagonal blocks' inverses into W's diagonal blocks (upper parts zero)

@@ -1669,12 +1669,11 @@ int coarsest_inverse(top_solver *s, cudaStream_t st)
 {
     const int64_t n = s->nC, nblk = (n + kDb - 1) / kDb;
     double *A = s->Ac;
-    static const bool attr = cudaFuncSetAttribute(chol_diag_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDiagSmem) == cudaSuccess &&
-                             cudaFuncSetAttribute(chol_panel_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPanelSmem) == cudaSuccess;
+    static const bool attr = chol_smem_attr() == cudaSuccess;
     if (!attr) { set_error("top_solver_assemble: shared memory of the coarsest factorisation"); return TOP_ERR_CUDA; }
     // Each step's trailing update is split: the next step's 128 columns first, on
     // the caller's stream, then the rest on a second stream, beside the next
-    // diagonal block (one CTA, 53 us) and panel, which touch other columns.
+    // diagonal block (one CTA, 37 us) and panel, which touch other columns.
     if (n > 2 * kPb && !s->auxStream) {
         CK(cudaStreamCreateWithFlags(&s->auxStream, cudaStreamNonBlocking));
         CK(cudaEventCreateWithFlags(&s->auxGo, cudaEventDisableTiming));
@@ -1688,10 +1687,10 @@ int coarsest_inverse(top_solver *s, cudaStream_t st)
         const int64_t rest = n - k0 - kPb;
         if (rest <= 0) break;
         const int nt = (int)((rest + kTileB - 1) / kTileB);
-        chol_panel_kernel<<<(unsigned)nt, kPanelThreads, kPanelSmem, st>>>(A, n, k0, s->Dc);
+        chol_panel(A, n, k0, s->Dc, s->numSMs, st);
         if (nt > kNext) CK(cudaEventRecord(s->auxGo, st));                 // the panel is complete
         if (restRuns) CK(cudaStreamWaitEvent(st, s->auxDone, 0));          // the previous step's updates of these columns
-        chol_trail_kernel<<<dim3((unsigned)nt, (unsigned)std::min(nt, kNext)), kTileThreads, 0, st>>>(A, n, k0, 0);
+        chol_next(A, n, k0, st);
         s->launches += 2;
         restRuns = nt > kNext;
         if (restRuns) {
