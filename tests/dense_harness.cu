@@ -39,17 +39,15 @@ int main(int argc, char **argv)
         for (int64_t k0 = 0; k0 < n; k0 += kPb) {
             chol_diag_kernel<<<1, kDiagThreads, kDiagSmem>>>(dA, n, k0, D, st);
             const int64_t rest = n - k0 - kPb;
-            if (rest <= 0) break;
-            const unsigned nt = (unsigned)((rest + kTileB - 1) / kTileB);
-            chol_panel(dA, n, k0, D, sms, 0);
-            chol_next(dA, n, k0, 0);
-            if (nt > 2) chol_trail_kernel<<<dim3(nt, nt - 2), kTileThreads>>>(dA, n, k0, 2);
+            if (rest > 0) {
+                const unsigned nt = (unsigned)((rest + kTileB - 1) / kTileB);
+                chol_panel(dA, n, k0, D, sms, 0);
+                chol_next(dA, n, k0, 0);
+                if (nt > 2) chol_trail_kernel<<<dim3(nt, nt - 2), kTileThreads>>>(dA, n, k0, 2);
+            }
+            if (sms != 12) inverse_columns(dA, W, I, D, n, k0, std::min<int64_t>(n, k0 + kPb), 0);
         }
-        place_dinv_kernel<<<(unsigned)((n + kDb - 1) / kDb), kDb * kDb>>>(D, W, n);
-        for (int64_t hs = kDb; hs < n; hs *= 2) {
-            const unsigned nodes = (unsigned)((n + 2 * hs - 1) / (2 * hs)), tiles = (unsigned)((hs + kTileB - 1) / kTileB);
-            for (int step = 0; step < 2; ++step) inv_level_kernel<<<dim3(tiles, tiles, nodes), kTileThreads>>>(dA, W, I, n, (int)hs, step);
-        }
+        if (sms == 12) inverse_columns(dA, W, I, D, n, 0, n, 0);       // both orders of the inversion
         const unsigned t = (unsigned)((n + kTileB - 1) / kTileB);
         dgemm_tile_kernel<true, true><<<dim3(t, t), kTileThreads>>>(I, n, W, n, W, n, (int)n, (int)n, (int)n, 0, 1, 1);
         int s = -1;

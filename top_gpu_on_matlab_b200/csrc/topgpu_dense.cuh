@@ -13,7 +13,8 @@
 //     summed from zero, as a sweep of one block at a time gives them;
 //   * W = L^-1 by 2x2 block inversion, [L11 0; L21 L22]^-1 =
 //     [W11 0; -W22 L21 W11  W22], bottom-up from the factorisation's
-//     diagonal blocks, every node of a level in one launch;
+//     diagonal blocks, each node as soon as its columns of L are complete, or
+//     after the factor every node of a level in one launch;
 //   * A^-1 = W^T W on the lower tiles, mirrored, skipping the zero blocks of W.
 //
 // Measured on one B200, factor and inverse (bit-identical to the sweep of one
@@ -35,6 +36,7 @@
 // instructions of 256 multiply-adds, against 16 multiply-adds a lane before.
 #pragma once
 #include <cuda_runtime.h>
+#include <algorithm>
 #include <cstdint>
 #include "topgpu_kernels.cuh"
 
@@ -172,14 +174,14 @@ wtw_packed_kernel(double *__restrict__ P, const double *__restrict__ W, int64_t 
 
 // One level of the bottom-up block inversion of a lower-triangular L (n x n):
 // node z covers rows [r0, r0 + 2 hs), r0 = 2 hs z, split at rh = r0 + hs; its
-// two products, over blockIdx.z:
+// two products, over blockIdx.z from node z0 on:
 //   step 0:  T = L21 W11      (T stored where W21 goes in Tb)
 //   step 1:  W21 = -W22 T
 // W11 and W22 are complete from the level below.
 __global__ void __launch_bounds__(kTileThreads)
-inv_level_kernel(const double *__restrict__ L, double *__restrict__ W, double *__restrict__ Tb, int64_t n, int hs, int step)
+inv_level_kernel(const double *__restrict__ L, double *__restrict__ W, double *__restrict__ Tb, int64_t n, int hs, int step, int z0)
 {
-    const int64_t r0 = (int64_t)blockIdx.z * 2 * hs, rh = r0 + hs;
+    const int64_t r0 = (int64_t)(z0 + blockIdx.z) * 2 * hs, rh = r0 + hs;
     if (rh >= n) return;
     const int64_t r1 = r0 + 2 * hs < n ? r0 + 2 * hs : n;
     const int s2 = (int)(r1 - rh);
@@ -587,13 +589,37 @@ inline cudaError_t chol_smem_attr()
     return e;
 }
 
-// copy the diagonal blocks' inverses into W's diagonal blocks (upper parts zero)
-__global__ void place_dinv_kernel(const double *__restrict__ Dinv, double *__restrict__ W, int64_t n)
+// copy the diagonal blocks' inverses from block b0 on into W's diagonal blocks (upper parts zero)
+__global__ void place_dinv_kernel(const double *__restrict__ Dinv, double *__restrict__ W, int64_t n, int64_t b0)
 {
-    const int64_t b = blockIdx.x;
+    const int64_t b = b0 + blockIdx.x;
     const int r = threadIdx.x % kDb, c = threadIdx.x / kDb;      // 32 x 32 threads
     const int64_t i = b * kDb + r, j = b * kDb + c;
     if (i < n && j < n) W[i + n * j] = Dinv[b * kDb * kDb + r + kDb * c];
+}
+// What columns c0 .. c - 1 of L add to W = L^-1 (W zero before the first; c0 a multiple
+// of 128; L complete in its columns before c): of every level, the products T of the
+// nodes whose left half, and W21 of the nodes that, end there.  Called after each step of
+// the factorisation on a stream beside it, this leaves the last rows' products for
+// after the factor; called once, for all columns, it takes each level in two launches.
+// Returns the launches.
+inline int inverse_columns(const double *L, double *W, double *T, const double *Dinv, int64_t n, int64_t c0, int64_t c, cudaStream_t st)
+{
+    int launches = 1;
+    place_dinv_kernel<<<(unsigned)((c - c0 + kDb - 1) / kDb), kDb * kDb, 0, st>>>(Dinv, W, n, c0 / kDb);
+    for (int64_t hs = kDb; hs < n; hs *= 2) {
+        const int64_t all = (n - hs + 2 * hs - 1) / (2 * hs);                // nodes with rows on both sides of their split
+        auto left = [&](int64_t e) { return e < hs ? 0 : std::min(all, (e - hs) / (2 * hs) + 1); };
+        auto whole = [&](int64_t e) { return e >= n ? all : std::min(all, e / (2 * hs)); };
+        const unsigned tiles = (unsigned)((hs + kTileB - 1) / kTileB);
+        for (int step = 0; step < 2; ++step) {
+            const int64_t z0 = step ? whole(c0) : left(c0), z1 = step ? whole(c) : left(c);
+            if (z1 <= z0) continue;
+            inv_level_kernel<<<dim3(tiles, tiles, (unsigned)(z1 - z0)), kTileThreads, 0, st>>>(L, W, T, n, (int)hs, step, (int)z0);
+            ++launches;
+        }
+    }
+    return launches;
 }
 
 }  // namespace topgpu
