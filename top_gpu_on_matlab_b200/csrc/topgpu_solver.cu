@@ -1633,6 +1633,10 @@ int build_tail(top_solver *s, cudaStream_t st)
 {
     s->tailReady = false;
     if (!tail_on(s)) return TOP_OK;
+    // the coarsest operator as a whole matrix: where it is kept as packed tiles
+    // (separate bodies, each as small as a coarsest cell, have both that many DOFs
+    // there and few enough a level up), s->Ainv holds the inversion's scratch instead
+    if (s->symPart) whole_inverse(s, st);
     const double *Mnext = s->Ainv;
     for (int l = s->nL - 2; l >= s->tailL; --l) {
         const size_t k = (size_t)(l - s->tailL);
@@ -1728,7 +1732,8 @@ int coarsest_inverse(top_solver *s, cudaStream_t st)
         CK(cudaStreamWaitEvent(st, s->invDone, 0));
     }
     // W^T W: whole, or as packed tiles over the factor, which is no longer needed.
-    // The persistent coarse V-cycle (an option) reads it whole.
+    // The persistent coarse V-cycle (an option) reads it whole; so does build_tail,
+    // which forms it for itself.
     const unsigned nt = (unsigned)((n + kTileB - 1) / kTileB);
     if (s->symPart) {
         wtw_packed_kernel<<<dim3(nt, nt), kTileThreads, 0, st>>>(s->Ac, s->Wc, n);
