@@ -277,8 +277,8 @@ __device__ __forceinline__ bool two_sums_last(double s1, double s2, double *part
 // scalar PCG pieces (one component)
 // The start, one launch: the nodal right-hand side b = sum of the (pre-scaled)
 // values of the node's elements (TOP_GPU.m:975-996), x = 0, r = b, z = M r, p = z
-// on every node of the grid (the vectors are zero elsewhere), ||b||, z.r and
-// the solve's state
+// on every node of the grid (the vectors are zero elsewhere: filter_apply clears
+// them after a solve that was not finite), ||b||, z.r and the solve's state
 __global__ void __launch_bounds__(256)
 fpcg_init_kernel(const double *__restrict__ eg, Geom g, const uint8_t *__restrict__ flags, double *__restrict__ x, double *__restrict__ r,
                  double *__restrict__ z, double *__restrict__ p, const double *__restrict__ invD, PcgState *st, double tol, int maxIT,
@@ -826,7 +826,13 @@ static int filter_apply(top_solver *s, const double *src, double *tar, int *itsO
     TOPGPU_COUNT_LAUNCH();
     CK(cudaGetLastError());
     if (itsOut) *itsOut = h.its;
-    if (h.status == TOP_ERR_NAN) { set_error("PDE filter: non-finite PCG scalar"); return TOP_ERR_NAN; }
+    if (h.status == TOP_ERR_NAN) {
+        // the update ran over every slot with a non-finite step length (0 * NaN):
+        // padding and guard slots, which the start does not write, go back to zero
+        for (double *q : {f.x, f.r, f.z, f.p}) CK(cudaMemsetAsync(q - kMargin, 0, sizeof(double) * g.cs, st));
+        set_error("PDE filter: non-finite PCG scalar");
+        return TOP_ERR_NAN;
+    }
     return TOP_OK;
 }
 
