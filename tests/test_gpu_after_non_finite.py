@@ -62,3 +62,48 @@ def test_filter(bad):
         _fails(lambda: s.filter(y))
         out, k = s.filter(x)
         assert k == its and torch.equal(out, ref)
+
+
+@pytest.mark.parametrize("mixed", [False, True])
+@pytest.mark.parametrize("bad", BAD[:2])
+def test_pcg_right_hand_side(mixed, bad):
+    m = _mesh()
+    fresh, s = _solver(m, mixed), _solver(m, mixed)
+    U0, its0, _ = fresh.pcg(0)
+    b = torch.zeros(s.numDOFs, dtype=torch.float64, device="cuda")
+    b[5 * 3 + 1] = bad
+    for _ in range(2):
+        _fails(lambda: s.pcg(b=b))
+        U, its, _ = s.pcg(0)
+        assert its == its0 and torch.equal(U, U0)
+
+
+@pytest.mark.parametrize("mixed", [False, True])
+def test_batched_pcg_warm_start(mixed):
+    """one of three load cases starts from a vector with a NaN"""
+    from top_gpu_on_matlab_b200._lib import TopGpuError
+    m = _mesh(3)
+    fresh, s = _solver(m, mixed), _solver(m, mixed)
+    U0, its0, _ = fresh.pcg_all()
+    W = torch.zeros_like(U0)
+    W[s.numDOFs + 11] = float("nan")
+    with pytest.raises(TopGpuError):
+        s.pcg_all(W)
+    U, its, _ = s.pcg_all()
+    assert its == its0 and torch.equal(U, U0)
+
+
+@pytest.mark.parametrize("mixed", [False, True])
+def test_density(mixed):
+    m = _mesh()
+    fresh, s = _solver(m, mixed), _solver(m, mixed)
+    x = _density(s)
+    y = x.clone()
+    y[7] = float("nan")
+    s.set_density(y)
+    _fails(s.assemble)
+    s.set_density(x)
+    s.assemble()
+    U0, its0, _ = fresh.pcg(0)
+    U, its, _ = s.pcg(0)
+    assert its == its0 and torch.equal(U, U0)

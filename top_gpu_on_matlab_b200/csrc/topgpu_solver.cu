@@ -2079,7 +2079,13 @@ int topgpu::pcg_block(top_solver *s, const double *bGrid, double *xg, int nrhs, 
         if (f.normB == 0.0) CK(cudaMemsetAsync(xg + k * nv - kMargin, 0, sizeof(double) * nv, st));
         if (itsOut) itsOut[k] = f.its;
         if (resOut) resOut[k] = f.resnorm;
-        if (f.status == TOP_ERR_NAN) { set_error("top_solver_pcg: non-finite PCG scalar at iteration %d", f.its); rc = TOP_ERR_NAN; }
+        if (f.status == TOP_ERR_NAN) {
+            // a non-finite step length went into every slot, and the first direction
+            // of the next solve is z + 0 p: back to the zeros of the allocation
+            if (rc != TOP_ERR_NAN) CK(clear_vectors(s));
+            set_error("top_solver_pcg: non-finite PCG scalar at iteration %d", f.its);
+            rc = TOP_ERR_NAN;
+        }
         else if (f.status == TOP_ERR_NOT_CONVERGED && rc == TOP_OK) {
             set_error("Exceed the maximum iterate numbers (residual %.4e)", f.resnorm); rc = TOP_ERR_NOT_CONVERGED;
         }

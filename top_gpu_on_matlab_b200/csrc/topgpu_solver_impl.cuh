@@ -256,6 +256,23 @@ inline void packed_op(top_solver *s, DevLevel &lv, const In &in, const Out &out,
 }  // namespace topgpu
 
 namespace topgpu {
+// The work vectors of PCG and the V-cycle as they were allocated: zero.  None
+// holds anything between two calls, but slots without an active node (padding,
+// guards, void layers) are not written by every kernel that relies on their zeros.
+inline cudaError_t clear_vectors(top_solver *s)
+{
+    cudaError_t e = cudaSuccess;
+    auto clear = [&](auto *v, int64_t cs) {
+        if (v && e == cudaSuccess) e = cudaMemsetAsync(v - kMargin, 0, sizeof(*v) * 3 * cs * s->kMax, s->st);
+    };
+    const int64_t cs0 = s->L[0].g.cs;
+    clear(s->r, cs0); clear(s->z, cs0); clear(s->z32, cs0); clear(s->pv, cs0); clear(s->v, cs0);
+    for (DevLevel &l : s->L) {
+        clear(l.r64, l.g.cs); clear(l.x64, l.g.cs); clear(l.t64, l.g.cs);
+        clear(l.r32, l.g.cs); clear(l.x32, l.g.cs); clear(l.t32, l.g.cs);
+    }
+    return e;
+}
 // y-epilogue applied to (K_0 in)(node) for every level-0 node, with the
 // level-0 kernel configured for precision T (topgpu_l0.cu)
 template <typename T, class In, class Out>
