@@ -107,3 +107,41 @@ def test_density(mixed):
     U0, its0, _ = fresh.pcg(0)
     U, its, _ = s.pcg(0)
     assert its == its0 and torch.equal(U, U0)
+
+
+@pytest.mark.parametrize("mixed", [False, True])
+def test_operators(mixed):
+    """The V-cycle and the product on a vector with a NaN, through the level-0
+    kernel that visits every layer; then through the one that leaves the void
+    layers out."""
+    m = _mesh()
+    out = []
+    for bad in (0.0, float("nan")):
+        s = _solver(m, mixed)
+        s.set_l0_kernel(False, 1, 16, 8, 12 * 148)
+        s.set_l0_kernel(True, 1, 16, 8, 12 * 148)
+        u = torch.from_numpy(np.random.default_rng(3).standard_normal(s.numDOFs)).cuda()
+        v = u.clone()
+        if bad != 0.0:
+            v[:] = bad
+        s.matvec(0, v), s.matvec(0, v, fp32=True), s.vcycle(v)
+        s.set_l0_kernel(False, 3, 16, 8, 12 * 148)
+        s.set_l0_kernel(True, 3, 16, 8, 12 * 148)
+        out.append([s.matvec(0, u), s.matvec(0, u, fp32=True), s.vcycle(u), s.pcg(0)[0]])
+    for a, b in zip(*out):
+        assert torch.equal(a, b)
+
+
+def test_single_product_before_a_double_vcycle():
+    """y = K u in single through a kernel that visits every layer, on a vector with
+    a NaN; then the FP64 V-cycle, whose kernel leaves the void layers out."""
+    m = _mesh()
+    out = []
+    for bad in (0.0, float("nan")):
+        s = _solver(m, False)
+        s.set_l0_kernel(True, 1, 16, 8, 12 * 148)
+        s.set_l0_kernel(False, 3, 16, 8, 12 * 148)
+        u = torch.from_numpy(np.random.default_rng(3).standard_normal(s.numDOFs)).cuda()
+        s.matvec(0, torch.full_like(u, bad), fp32=True)
+        out.append(s.vcycle(u))
+    assert torch.equal(*out)

@@ -383,6 +383,9 @@ int set_l0_kernel(top_solver *s, int p, int kind, int ty, int tx, int ctas)
     if (kind == 3) {
         const int rc = l0_active_ranges(s, k, ty, tx);
         if (rc != TOP_OK) { k.kind = 0; ++s->opGen; return rc; }
+        // the layers it leaves out have to be zero: another kind, which writes
+        // them, may have left 0 * NaN there
+        if (k.rng && clear_vectors(s) != cudaSuccess) return TOP_ERR_CUDA;
     }
     k.kind = kind; k.ty = ty; k.tx = tx; k.ctas = ctas;
     ++s->opGen;

@@ -1822,9 +1822,13 @@ extern "C" int top_solver_matvec(top_solver *s, int level, const double *u, doub
     if (level == s->nL - 1 && level > 0) { set_error("top_solver_matvec: the coarsest level is solved directly"); return TOP_ERR_ARGS; }
     DevLevel &d = s->L[level];
     const Reduce none{nullptr, nullptr, nullptr};
+    double *yg = d.t64;
     if (fp32) {                      // the operand rounded to FP32 once (as the V-cycle holds it)
+        // not into level 0's t64, the FP64 V-cycle's: where this precision's kernel writes
+        // void layers that the other one leaves out, 0 * NaN would stay in it
+        if (level == 0) yg = s->tmp;
         CK(to_grid(s, level, u, d.x32));
-        level_op<float>(s, level, VecIn<float, float>{d.x32, d.g.cs}, StoreOut<float, double>{d.t64, d.g.cs}, none, nullptr);
+        level_op<float>(s, level, VecIn<float, float>{d.x32, d.g.cs}, StoreOut<float, double>{yg, d.g.cs}, none, nullptr);
     } else {
         CK(to_grid(s, level, u, d.x64));
         if (level == 0) {            // straight to compact order: no grid vector written and read back (17 us on 96x192x96)
@@ -1834,9 +1838,9 @@ extern "C" int top_solver_matvec(top_solver *s, int level, const double *u, doub
             CK(cudaStreamSynchronize(s->st));          // a voxel level 0 has no bounded waits to report
             return TOP_OK;
         }
-        level_op<double>(s, level, VecIn<double, double>{d.x64, d.g.cs}, StoreOut<double, double>{d.t64, d.g.cs}, none, nullptr);
+        level_op<double>(s, level, VecIn<double, double>{d.x64, d.g.cs}, StoreOut<double, double>{yg, d.g.cs}, none, nullptr);
     }
-    grid_to_compact_kernel<double, double><<<nb256(d.Nn), 256, 0, s->st>>>(d.t64, y, d.nodeGrid, d.Nn, d.g.cs);
+    grid_to_compact_kernel<double, double><<<nb256(d.Nn), 256, 0, s->st>>>(yg, y, d.nodeGrid, d.Nn, d.g.cs);
     TOPGPU_COUNT_LAUNCH();
     CKL();
     return op_err_status(s);

@@ -857,7 +857,8 @@ __device__ __forceinline__ void l0d_march_c2(const WalshParam<float> &B, const I
 
 // rng (may be null): a tile's layers outside [x, y) hold no active node and are not
 // visited -- their outputs are zero and stay so, since every vector is zero
-// there from its allocation.  The CTAs' shares stay those of all layers, so
+// there from its allocation (clear_vectors puts that back: when a kind that visits
+// them gives way to this one, and after a solve that was not finite).  The CTAs' shares stay those of all layers, so
 // that a fused dot product adds the same terms in the same order; the several
 // waves of CTAs even out what the shares then differ by.  Irregular domain in a
 // 96x192x96 grid (a third solid), four load cases: 1040 -> 652 us a PCG iteration
