@@ -395,18 +395,23 @@ __device__ __forceinline__ void sub_to_fine(int64_t i, int ny, int nx, int &y, i
     y = 4 * ey + (q & 3); x = 4 * ex + ((q >> 2) & 3); z = 4 * ez + (q >> 4);
 }
 // the correlation's operand: the fine grid with x fastest inside a margin of
-// R zeros (kSfRows - 1 more past the last y, for the last thread's rows)
+// zeros (kSfRows - 1 more past the last y, for the last thread's rows), the taps'
+// reach or, where that is more than the grid's, what two of its voxels can be apart
 constexpr int kSfRows = 8;
 struct SfGeom {
-    int fy, fx, fz, R;
-    __host__ __device__ int px() const { return fx + 2 * R; }
-    __host__ __device__ int py() const { return fy + 2 * R + kSfRows - 1; }
-    __host__ __device__ int64_t size() const { return (int64_t)px() * py() * (fz + 2 * R); }
-    // first tap of output (y, x, z): operand entry (y - R, x - R, z - R)
+    int fy, fx, fz, ry, rx, rz;
+    __host__ __device__ SfGeom(int y, int x, int z, int R)
+        : fy(y), fx(x), fz(z), ry(R < y ? R : y - 1), rx(R < x ? R : x - 1), rz(R < z ? R : z - 1) {}
+    __host__ __device__ int px() const { return fx + 2 * rx; }
+    __host__ __device__ int py() const { return fy + 2 * ry + kSfRows - 1; }
+    __host__ __device__ int64_t size() const { return (int64_t)px() * py() * (fz + 2 * rz); }
+    // first tap of output (y, x, z): operand entry (y - ry, x - rx, z - rz)
     __host__ __device__ int64_t at(int y, int x, int z) const { return x + (int64_t)px() * (y + (int64_t)py() * z); }
+    // taps [2 rz + 1][2 rx + 1][2 ry + 1], y fastest
+    __host__ __device__ int64_t tap(int y, int x, int z) const { return y + (int64_t)(2 * ry + 1) * (x + (int64_t)(2 * rx + 1) * z); }
 };
 // mode 0: g = in ./ Hs (sensitivities), mode 1: g = in (densities); Hs in the
-// element-major order of in (mode 0 with Hs null: ones)
+// element-major order of in (not read in mode 1)
 __global__ void sfilt_gather_kernel(const double *__restrict__ in, const double *__restrict__ Hs, int mode, int ny, int nx,
                                     SfGeom s, int64_t n, double *__restrict__ g)
 {
@@ -414,18 +419,22 @@ __global__ void sfilt_gather_kernel(const double *__restrict__ in, const double 
     if (i >= n) return;
     int y, x, z;
     sub_to_fine(i, ny, nx, y, x, z);
-    g[s.at(y + s.R, x + s.R, z + s.R)] = mode == 0 ? in[i] / Hs[i] : in[i];
+    g[s.at(y + s.ry, x + s.rx, z + s.rz)] = mode == 0 ? in[i] / Hs[i] : in[i];
 }
 // t = imfilter(g, h): correlation, zero outside (the kernel is symmetric), and
-// out = t (mode 0) or t ./ Hs (mode 1), element-major.  FP64-issue bound: (2R+1)^3
-// multiply-adds an output.  A thread forms YB outputs consecutive in y with its
+// out = t (mode 0) or t ./ Hs (mode 1), element-major.  FP64-issue bound: up to
+// (2R+1)^3 multiply-adds an output.  A thread forms YB outputs consecutive in y with its
 // lanes along x (coalesced operand rows); for each (dz, dx) it slides over the
-// 2R + YB operand rows in groups of four taps, so a group costs 4 operand and
-// 4 tap loads for 4 YB multiply-adds; the loads' L1 wavefronts bound it now.  On
-// the 40x240x40 fine grid at R = 6: 633 us (one output a thread, two loads a
-// multiply-add behind bounds checks) -> 219 us, the whole filter 638 -> 240 us.
-// The multiply-adds run in the order dz, dx, dy ascending; taps outside the
-// grid read the zero margin.
+// operand rows in groups of four taps, so a group costs 4 operand and
+// 4 tap loads for 4 YB multiply-adds; the loads' L1 wavefronts bound it now.
+// Planes and rows outside the grid are left out (lanes of a warp mostly share z
+// and y, so that costs no divergence; in x, where they differ, such taps read the
+// zero margin), and the taps reach no further than two voxels of the grid are
+// apart: a radius of the grid's size costs no more than its voxels.  The whole
+// filter, one output a thread with two loads a multiply-add behind bounds checks ->
+// all taps of every output -> this: 40x240x40 fine grid, R = 6 640 -> 240 -> 216 us;
+// R = 47 94.9 -> 120.7 -> 17.9 ms; 24x64x24, R = 31 5.4 -> 17.7 -> 2.5 ms.
+// The multiply-adds run in the order dz, dx, dy ascending.
 template <int YB>
 __global__ void __launch_bounds__(128)
 sfilt_conv_kernel(const double *__restrict__ g, const double *__restrict__ h, SfGeom s, const double *__restrict__ Hs, int mode,
@@ -435,14 +444,18 @@ sfilt_conv_kernel(const double *__restrict__ g, const double *__restrict__ h, Sf
     const int ng = (s.fy + YB - 1) / YB;
     if (k >= (int64_t)s.fx * ng * s.fz) return;
     const int x = (int)(k % s.fx), y0 = (int)((k / s.fx) % ng) * YB, z = (int)(k / ((int64_t)s.fx * ng));
-    const int w = 2 * s.R + 1, px = s.px();
+    const int px = s.px();
+    // taps whose operand plane (z) or rows (y, of any of the YB outputs) are in the grid
+    const int zb = max(0, s.rz - z), ze = min(2 * s.rz + 1, s.fz + s.rz - z);
+    const int yb = max(0, s.ry - y0 - (YB - 1)), w = min(2 * s.ry + 1, s.fy + s.ry - y0) - yb;
     double acc[YB];
 #pragma unroll
     for (int u = 0; u < YB; ++u) acc[u] = 0.0;
-    for (int dz = 0; dz < w; ++dz)
-        for (int dx = 0; dx < w; ++dx) {
-            const double *gr = g + s.at(y0, x + dx, z + dz);
-            const double *hr = h + w * (dx + w * dz);
+    g += s.at(y0 + yb, x, z + zb);
+    h += s.tap(yb, 0, zb);
+    for (int dz = zb; dz < ze; ++dz, g += s.at(0, 0, 1) - (2 * s.rx + 1))
+        for (int dx = 0; dx < 2 * s.rx + 1; ++dx, ++g, h += 2 * s.ry + 1) {
+            const double *gr = g, *hr = h;
             double win[YB + 3];
 #pragma unroll
             for (int u = 0; u < YB - 1; ++u) win[u] = gr[(int64_t)px * u];
@@ -852,7 +865,7 @@ extern "C" int top_solver_filter(top_solver *s, const double *src, double *tar, 
 static void sfilt_conv(top_solver *s, const double *Hs, int mode, double *out)
 {
     SFilterState &f = opt(s).sf;
-    const SfGeom sg{f.fy, f.fx, f.fz, f.R};
+    const SfGeom sg(f.fy, f.fx, f.fz, f.R);
     const int64_t cols = (int64_t)f.fx * f.fz, n8 = cols * ((f.fy + 7) / 8), n4 = cols * ((f.fy + 3) / 4);
     if (n8 >= (int64_t)s->numSMs * 4 * 2 * 32)
         sfilt_conv_kernel<8><<<(unsigned)((n8 + 127) / 128), 128, 0, s->st>>>(f.g, f.h, sg, Hs, mode, s->nely, s->nelx, out);
@@ -870,25 +883,24 @@ static int sfilter_setup(top_solver *s, double rMin)
     }
     const double r = 4.0 * rMin;
     f.R = (int)std::ceil(r) - 1;
-    const int w = 2 * f.R + 1;
     f.fy = 4 * s->nely; f.fx = 4 * s->nelx; f.fz = 4 * s->nelz;
     const int64_t N = (int64_t)f.fy * f.fx * f.fz;
     if (!f.Hs) {
         f.Hs = s->dalloc<double>(N);
         if (!f.Hs) { set_error("super-element filter: out of device memory"); return TOP_ERR_NOMEM; }
     }
-    std::vector<double> h((size_t)w * w * w);
-    for (int dz = -f.R; dz <= f.R; ++dz)
-        for (int dx = -f.R; dx <= f.R; ++dx)
-            for (int dy = -f.R; dy <= f.R; ++dy) {
+    const SfGeom sg(f.fy, f.fx, f.fz, f.R);
+    std::vector<double> h((size_t)sg.tap(0, 0, 2 * sg.rz + 1));
+    for (int dz = -sg.rz; dz <= sg.rz; ++dz)
+        for (int dx = -sg.rx; dx <= sg.rx; ++dx)
+            for (int dy = -sg.ry; dy <= sg.ry; ++dy) {
                 const double v = r - std::sqrt(double(dx * dx + dy * dy + dz * dz));
-                h[(dy + f.R) + w * ((dx + f.R) + w * (dz + f.R))] = v > 0 ? v : 0.0;
+                h[(size_t)sg.tap(dy + sg.ry, dx + sg.rx, dz + sg.rz)] = v > 0 ? v : 0.0;
             }
     f.ready = false;
     if (f.h) cudaFree(f.h);
     if (f.g) cudaFree(f.g);
     f.h = f.g = nullptr;
-    const SfGeom sg{f.fy, f.fx, f.fz, f.R};
     if (cudaMalloc(&f.h, sizeof(double) * h.size()) != cudaSuccess) { f.h = nullptr; return TOP_ERR_NOMEM; }
     if (cudaMalloc(&f.g, sizeof(double) * sg.size()) != cudaSuccess) { f.g = nullptr; return TOP_ERR_NOMEM; }
     CK(cudaMemcpyAsync(f.h, h.data(), sizeof(double) * h.size(), cudaMemcpyHostToDevice, s->st));
@@ -909,7 +921,7 @@ static int sfilter_apply(top_solver *s, const double *in, double *out, int mode)
 {
     SFilterState &f = opt(s).sf;
     const int64_t n = 64 * s->L[0].Ne;
-    const SfGeom sg{f.fy, f.fx, f.fz, f.R};
+    const SfGeom sg(f.fy, f.fx, f.fz, f.R);
     sfilt_gather_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s->st>>>(in, f.Hs, mode, s->nely, s->nelx, sg, n, f.g);
     TOPGPU_COUNT_LAUNCH();
     sfilt_conv(s, f.Hs, mode, out);
