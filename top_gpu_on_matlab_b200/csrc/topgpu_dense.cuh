@@ -39,6 +39,7 @@
 #include <algorithm>
 #include <cstdint>
 #include "topgpu_kernels.cuh"
+#include "topgpu_grid.cuh"
 
 namespace topgpu {
 
@@ -220,22 +221,34 @@ inv_level_kernel(const double *__restrict__ L, double *__restrict__ W, double *_
 // tells the others on the column's own mbarrier (ready[j], one phase a block; no
 // cycles lost on the chain, where a barrier they all meet at cost 70 a column).
 // a[i] is entry (r, j + i) while the owner eliminates column j, so the loop body is
-// the same for every column and stays in the instruction cache.  status: set when a
-// pivot is not positive (the pivot is then taken as 1).
+// the same for every column and stays in the instruction cache.  status: kCholPivot
+// is set when a pivot is not positive (the pivot is then taken as 1), kCholWait
+// when a wait for a column ran out.
+constexpr int kCholPivot = 1, kCholWait = 2;
 constexpr int kCholLd = kDb + 2;         // column j of L from row j + 1 on: sL[j][i] = L[j + 1 + i][j]
 constexpr int kCholWarps = 6;
 __device__ __forceinline__ void chol_ready(uint64_t *ready)
 {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" :: "r"((unsigned)__cvta_generic_to_shared(ready)) : "memory");
 }
-// bounded: past the limit the factor is flagged and the warp goes on
+// Bounded (one second): past it the status says so, the warp goes on, and waits
+// that do not end at once give up from then on.  The clock and the status are
+// looked at every 64th try, so a wait that ends costs its tries alone.
 __device__ __forceinline__ void chol_await(uint64_t *ready, int phase, int *status)
 {
     const unsigned a = (unsigned)__cvta_generic_to_shared(ready);
-    unsigned ok = 0;
-    for (int tries = 0; !ok && tries < (1 << 20); ++tries)
+    auto over = [&] {
+        unsigned ok;
         asm volatile("{.reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p;}" : "=r"(ok) : "r"(a), "r"(phase) : "memory");
-    if (!ok) atomicExch(status, 1);
+        return ok != 0;
+    };
+    if (over()) return;
+    const uint64_t t0 = bulk::now_ns();
+    for (unsigned tries = 1; !over(); ++tries)
+        if (tries % 64 == 0 && ((*(volatile int *)status & kCholWait) || bulk::now_ns() - t0 > bulk::kWaitNs)) {
+            atomicOr(status, kCholWait);
+            return;
+        }
 }
 __device__ __forceinline__ void chol_block_warps(int w, double *S, int ld, double (*sL)[kCholLd], double *sInv, double *Ds, int ldd, uint64_t *ready, int phase, int *status)
 {
@@ -279,7 +292,7 @@ __device__ __forceinline__ void chol_block_warps(int w, double *S, int ld, doubl
                 if (i + 1 < 8) a[i] = fma(-l, lc.y, a[i + 1]);
             }
         }
-        if (bad && r == 0) atomicExch(status, 1);
+        if (bad && r == 0) atomicOr(status, kCholPivot);
     } else {
         const int h = r >> 4, c = (r & 15) + 16 * (w - 4);
         double x[kDb / 2];               // x[i] = entry (j + 2 i + h, c) of W at even steps j
@@ -337,7 +350,7 @@ constexpr size_t kDiagSmem = sizeof(double) * (kPb * kDiagLd + kDb * kCholLd + k
 // one SM's FP64 rate.  L over A's lower part,
 // the 32 x 32 diagonal blocks' inverses to Dinv (rows / columns past n the identity).
 // Between two 32-column blocks only the next diagonal block is brought up to
-// date; the other updates are the remaining warps' while five factor it.
+// date; the other updates are the remaining warps' while six factor it.
 __global__ void __launch_bounds__(kDiagThreads)
 chol_diag_kernel(double *A, int64_t n, int64_t k0, double *Dinv, int *status)
 {

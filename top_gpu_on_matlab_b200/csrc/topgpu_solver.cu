@@ -1549,7 +1549,7 @@ extern "C" int top_solver_set_density(top_solver *s, const double *x, int where)
 // Cholesky factor and explicit inverse of the coarsest matrix s->Ac (n x n,
 // column-major): L over Ac's lower triangle, W = L^-1 in s->Wc, A^-1 in
 // s->Ainv (which also serves as the product scratch of the inversion);
-// a non-positive pivot sets s->zeroDone[1]
+// a non-positive pivot sets kCholPivot in s->zeroDone[1], a wait that ran out kCholWait
 namespace {
 // C = A B^T on the tiled tensor-core product: (ta, tb) as dgemm_tile_kernel's;
 // lower / mirror / kFromTile likewise
@@ -1793,6 +1793,7 @@ extern "C" int top_solver_assemble(top_solver *s)
     int flag = 0;
     CK(cudaMemcpyAsync(&flag, s->zeroDone + 1, sizeof(int), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
+    if (flag & kCholWait) { set_error("top_solver_assemble: a wait in the coarsest factorisation ran out"); return TOP_ERR_CUDA; }
     if (flag) { set_error("top_solver_assemble: coarsest matrix is not positive definite"); return TOP_ERR_NAN; }
     { const int rc = build_tail(s, st); if (rc) return rc; }
     s->assembled = true;
