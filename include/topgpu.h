@@ -87,7 +87,8 @@ int top_assemble_ks_level2(void *Ks, const int32_t *upMap, const void *eleModulu
  * GPU, held until exit); nCh is limited to 64 (TOP_ERR_SHAPE above that).
  * The first call on a device, and the first after its context was replaced
  * (cudaDeviceReset), resolves the array's address (make it before any stream
- * capture); concurrent calls on one device race -- serialise them. */
+ * capture); concurrent calls in double on one device race -- serialise them
+ * (calls in single use no scratch). */
 int top_assemble_ks_level2_noalloc(void *Ks, const int32_t *upMap, const void *eleModulus,
                                    const void *K0, const void *Pch, const int32_t *mapUnique,
                                    const void *uniqueFree, const void *uniqueFixed,

@@ -400,9 +400,10 @@ extern "C" int top_assemble_ks_level2_super(void *Ks, const int32_t *upMap, cons
 //    context was replaced, e.g. by cudaDeviceReset) resolves the arrays'
 //    device addresses with cudaGetSymbolAddress, with that device current;
 //    make that call before any stream capture on that device;
-//  * all calls share the arrays and each call clears the part it reads, so
-//    calls that run concurrently on the GPU (different streams or threads)
-//    race -- serialise them.
+//  * all calls in double share the array and each clears it, so such calls
+//    that run concurrently on the GPU (different streams or threads) race --
+//    serialise them.  Calls in single take no scratch: every CTA forms the part
+//    of Q it multiplies by.
 namespace {
 constexpr int kNoAllocMaxChildren = 64;
 constexpr int kNoAllocMaxDevices = 64;
@@ -473,17 +474,20 @@ extern "C" int top_assemble_ks_level2_noalloc(void *Ks, const int32_t *upMap, co
     if (!Ks || !upMap || !eleModulus || !K0 || !Pch) { set_error("%s:Input null pointer", N); return TOP_ERR_ARGS; }
     const int hasFixed = (nUnique > 0 && mapUnique && uniqueFree && uniqueFixed) ? 1 : 0;
     cudaStream_t st = S(stream);
-    NoAllocScratch sc;
-    int rc = noalloc_scratch(&sc, N);
-    if (rc) return rc;
-    // the GEMM loads all 64 rows of Q and multiplies rows nCh..63 by zero:
-    // clear them all, so that no value left by an earlier call (NaN or Inf
-    // included) reaches this call's result
-    TOP_CUDA_CHECK(cudaMemsetAsync(sc.Q, 0, sizeof(double) * 576 * kNoAllocMaxChildren, st), N);
     const int64_t nu = hasFixed ? nUnique : 0;
-    rc = dtype == TOP_F64
-        ? level2_typed<double>(Ks, upMap, eleModulus, K0, Pch, mapUnique, uniqueFree, uniqueFixed, nElem, nCh, nu, sc.Q, st)
-        : level2_typed<float>(Ks, upMap, eleModulus, K0, Pch, mapUnique, uniqueFree, uniqueFixed, nElem, nCh, nu, sc.Q, st);
+    int rc;
+    if (dtype == TOP_F64) {
+        NoAllocScratch sc;
+        rc = noalloc_scratch(&sc, N);
+        if (rc) return rc;
+        // the GEMM loads all 64 rows of Q and multiplies rows nCh..63 by zero:
+        // clear them all, so that no value left by an earlier call (NaN or Inf
+        // included) reaches this call's result
+        TOP_CUDA_CHECK(cudaMemsetAsync(sc.Q, 0, sizeof(double) * 576 * kNoAllocMaxChildren, st), N);
+        rc = level2_typed<double>(Ks, upMap, eleModulus, K0, Pch, mapUnique, uniqueFree, uniqueFixed, nElem, nCh, nu, sc.Q, st);
+    } else {                         // no scratch: concurrent calls in single share nothing
+        rc = level2_typed<float>(Ks, upMap, eleModulus, K0, Pch, mapUnique, uniqueFree, uniqueFixed, nElem, nCh, nu, nullptr, st);
+    }
     if (rc) { set_error("%s:CUDA launch failed: %s", N, cudaGetErrorString(cudaGetLastError())); return rc; }
     TOP_CUDA_CHECK(cudaGetLastError(), N);
     TOP_CUDA_CHECK(cudaStreamSynchronize(st), N);
