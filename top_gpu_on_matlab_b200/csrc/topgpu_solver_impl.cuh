@@ -50,9 +50,9 @@ struct top_solver {
     bool useGraphs = true;
     bool coarseLanes = std::getenv("TOPGPU_COARSE_LANES") != nullptr;   // 8-lanes-per-node coarse kernel
     int coarsePersistent = 0;        // levels from 1 (1) or from 2 (2) down of the V-cycle in one cooperative launch; 0 off
-    // coarse levels with at least this many packed tiles take the two-pass
-    // product (element outputs, then node sums; identical results)
-    int coarseTwoPassMin = std::getenv("TOPGPU_COARSE_TWOPASS_MIN") ? std::atoi(std::getenv("TOPGPU_COARSE_TWOPASS_MIN")) : 0;
+    // levels with at least this many packed tiles take the two-pass product
+    // (element outputs, then node sums; the same sums); negative: packed_op's rule
+    int coarseTwoPassMin = std::getenv("TOPGPU_COARSE_TWOPASS_MIN") ? std::atoi(std::getenv("TOPGPU_COARSE_TWOPASS_MIN")) : -1;
     bool pdl = std::getenv("TOPGPU_NO_PDL") == nullptr;
     // span-4 transfers read and write four fine y slots as one aligned vector
     // (identical results; TOPGPU_NO_VEC4 selects the per-slot kernels)
@@ -227,18 +227,31 @@ inline int coarse_elem_occ()
 }
 // y-epilogue applied to (K in)(node) for every node of a level with packed
 // element matrices, nv right-hand sides in one launch (vectors at the
-// functors' strides): the two passes, or the one-pass tile kernel where the
-// level has fewer tiles than the solver's threshold (the same sums).  At level
-// 0 of the 10x60x10 super-element model (FP64) the two passes take 9.7 + 5 to 7
-// us a product under ncu against 22 to 30 us for the tile kernel, which waits on
-// 72 scattered loads a thread; a PCG iteration 88.5 -> 82.5 us.
+// functors' strides): two passes, or the one-pass tile kernel (the same sums;
+// a fused dot product adds them in another grouping).  At level 0 of the 10x60x10
+// super-element model (FP64) the two passes take 9.7 + 5 to 7 us a product under
+// ncu against 22 to 30 us for the tile kernel, which waits on 72 scattered loads a
+// thread; a PCG iteration 88.5 -> 82.5 us.
+// Where the tile kernel's CTAs are one resident wave (four an SM) that wait is paid
+// once, and the second launch and the element outputs cost more: level 0 takes
+// one pass up to there, in single over all right-hand sides (in double the outputs
+// weigh twice, and more right-hand sides do not move the line).  A PCG
+// iteration on i x j x k super elements (tile CTAs a right-hand side), one / two
+// passes: FP64 10x20x13 (272) 63.1 / 69.1 us, 10x40x10 (442) 69.7 / 76.8, 10x48x10
+// (527) 72.3 / 76.4, 10x52x10 (612) 84.7 / 82.1, 16x64x16 (697) 87.9 / 81.7; with
+// four right-hand sides 272 92.3 / 103.4, 527 134.4 / 138.3, 612 155.8 / 147.8.
+// FP32 V-cycle: 442 63.2 / 67.2, 527 66.3 / 66.4, 612 76.5 / 72.3, two right-hand
+// sides 225 66.4 / 69.2, 357 75.6 / 73.1.
 template <typename T, class In, class Out>
 inline void packed_op(top_solver *s, DevLevel &lv, const In &in, const Out &out, Reduce red, const int *done, int nv)
 {
     int t0 = 0, nt = 0;
     coarse_elem_tiles(lv.g, t0, nt);
     T *W = wbuf<T>(lv);
-    if (W && s->opErr && nt > 0 && nt >= s->coarseTwoPassMin && coarse_elem_occ<T, In>() > 0) {
+    const dim3 one = coarse_tile_grid(lv.g);
+    const int64_t oneCtas = (int64_t)one.x * one.y * (sizeof(T) == 4 ? nv : 1);
+    const bool oneWave = s->coarseTwoPassMin < 0 && &lv == &s->L[0] && oneCtas <= 4 * (int64_t)s->numSMs;
+    if (W && s->opErr && nt > 0 && nt >= s->coarseTwoPassMin && !oneWave && coarse_elem_occ<T, In>() > 0) {
         const int64_t wvs = w_alloc_vals(lv.g.cs);
         const unsigned ctas = (unsigned)std::min<int64_t>(nt, (int64_t)s->numSMs * coarse_elem_occ<T, In>());
         launch_k(s, coarse_elem_kernel<T, In>, dim3(ctas, (unsigned)nv), kElemThreads, CoarseElem<T>::kSmem, s->st,
@@ -248,8 +261,7 @@ inline void packed_op(top_solver *s, DevLevel &lv, const In &in, const Out &out,
         launch_k(s, coarse_gather_kernel<T, Out>, dim3((unsigned)lv.g.nbx, (unsigned)lv.g.NZ, (unsigned)nv), kNodeThreads, 0, s->st,
                  out, W, wvs, lv.g, red, done);
     } else {
-        dim3 gr = coarse_tile_grid(lv.g); gr.z = (unsigned)nv;
-        launch_k(s, coarse_tile_kernel<T, In, Out>, gr, dim3(kCoarseTileX, 8), 0, s->st, in, out, ks_packed<T>(lv), lv.g, red, done);
+        launch_k(s, coarse_tile_kernel<T, In, Out>, dim3(one.x, one.y, (unsigned)nv), dim3(kCoarseTileX, 8), 0, s->st, in, out, ks_packed<T>(lv), lv.g, red, done);
     }
     TOPGPU_COUNT_LAUNCH();
 }
