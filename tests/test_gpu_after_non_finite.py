@@ -11,6 +11,11 @@ pytestmark = pytest.mark.gpu
 BAD = [float("nan"), float("inf"), 1e200]      # 1e200: finite, its square is not
 
 
+@pytest.fixture(autouse=True)
+def _void_left_out(monkeypatch):
+    monkeypatch.setenv("TOPGPU_VOID_MIN_SLOTS", "0")       # the models are small
+
+
 def _mesh(loads=1):
     from top_gpu_on_matlab_b200.fea import Mesh
     mask = np.zeros((18, 40, 20), bool)

@@ -311,10 +311,11 @@ int tc_selftest(top_solver *s, const top_solver::L0Kernel &cand)
 }
 }  // namespace
 
-// kind 3's ranges of active layers (kept null where no tile leaves any out)
+// kind 3's ranges of active layers (kept null on small grids and where no tile leaves any out)
 static int l0_active_ranges(top_solver *s, top_solver::L0Kernel &k, int ty, int tx)
 {
     const Geom &g = s->L[0].g;
+    if (s->L[0].ng < s->voidMinSlots) return TOP_OK;
     const int tiles = walsh_tiles(g, ty, tx);
     int2 *rng = nullptr;
     if (cudaMalloc(&rng, sizeof(int2) * (size_t)tiles) != cudaSuccess) return TOP_ERR_NOMEM;

@@ -1081,7 +1081,7 @@ extern "C" int top_solver_create(const top_mesh *mesh, const top_solver_params *
                     if (fl[(size_t)k]) { ch.push_back((int32_t)c); break; }
             }
             const int64_t whole = (3 * cs + kChunk - 1) / kChunk;
-            if ((int64_t)ch.size() * 3 * 10 > whole * 9) {      // under a tenth left out: the whole range
+            if (d.ng < s->voidMinSlots || (int64_t)ch.size() * 3 * 10 > whole * 9) {      // small, or under a tenth left out: the whole range
                 s->nChunks = (int)((whole + 2) / 3);
             } else {
                 s->nChunks = (int)ch.size();

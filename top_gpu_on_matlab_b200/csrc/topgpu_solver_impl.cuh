@@ -80,6 +80,13 @@ struct top_solver {
     int32_t *nodeOf = nullptr;       // level-0 grid slot -> compact node, 1-based (0: none), from the array's margin on
     // chunks of the level-0 vectors that the PCG vector kernels visit (ChunkList; null: all of them)
     int32_t *chunks = nullptr; int nChunks = 0;
+    // Level-0 grids of at least this many slots leave void layers (L0Kernel::rng) and
+    // chunks out.  Below, an iteration is launches and latency, and the lists' own loads
+    // come on top.  A PCG iteration without / with both on ragged boxes (slots), FP64:
+    // 20x53x16 (31 k) 60.3 / 62.2 us, 18x30x33 (42 k) 62.9 / 63.6, 20x60x20 (51 k)
+    // 69.3 / 63.8, 25x50x26 (74 k) 80.6 / 75.2; mixed: 16x24x17 (15 k) 38.9 / 41.2,
+    // 42 k 44.5 / 45.2, 51 k 47.5 / 45.0, 74 k 69.6 / 64.6.
+    int64_t voidMinSlots = std::getenv("TOPGPU_VOID_MIN_SLOTS") ? std::atoll(std::getenv("TOPGPU_VOID_MIN_SLOTS")) : 48 * 1024;
     int numSMs = 148;
     L0Kernel l0k[2];                 // [0] FP64, [1] FP32
     L0Kernel l0kFallback;            // kind 6 with a converting operand: the direct-load kind, 16 x 8
