@@ -1181,9 +1181,7 @@ extern "C" int top_solver_create(const top_mesh *mesh, const top_solver_params *
         l0.KsC = s->dalloc<double>((size_t)M0.Ne * 576);
         l0.KsP64 = s->ksalloc<double>(l0.g.cs);
         l0.KsP32 = s->ksalloc<float>(l0.g.cs);
-        l0.W64 = s->walloc<double>(l0.g.cs, s->kMax);    // element outputs of the two-pass product
-        l0.W32 = s->walloc<float>(l0.g.cs, s->kMax);
-        if (!s->Esub || !s->stage || !s->Imat || !l0.KsC || !l0.KsP64 || !l0.KsP32 || !l0.W64 || !l0.W32) return fail("out of device memory");
+        if (!s->Esub || !s->stage || !s->Imat || !l0.KsC || !l0.KsP64 || !l0.KsP32) return fail("out of device memory");
         cudaMemcpy(s->Imat, mesh->I_mat.data(), sizeof(double) * 576 * 64, cudaMemcpyHostToDevice);
     }
     s->uFixed = s->dalloc<double>((size_t)576 * s->nU);
@@ -1397,6 +1395,14 @@ extern "C" int top_solver_create(const top_mesh *mesh, const top_solver_params *
             s->numSMs = nsm;
     }
     coarse_elem_setup();
+    if (s->super) {      // element outputs of the two-pass product, after all else: without them it takes one pass
+        const bool mixed = s->p.precision == TOP_PREC_MIXED, outer32 = s->p.outerFP32 != 0;
+        // batches run in the V-cycle's and the outer product's precision, single products in both
+        const int n64 = mixed && outer32 ? 1 : s->kMax, n32 = mixed || outer32 ? s->kMax : 1;
+        if (!level0_one_wave<double>(s, l0, n64)) l0.W64 = s->walloc<double>(l0.g.cs, n64);
+        if (!level0_one_wave<float>(s, l0, n32)) l0.W32 = s->walloc<float>(l0.g.cs, n32);
+        (void)cudaGetLastError();
+    }
     // level-0 products in the Walsh basis where Ke allows it (voxel mode)
     if (s->super) s->walshOK = false;
     if (s->walshOK)

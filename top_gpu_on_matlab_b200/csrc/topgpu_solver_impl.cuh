@@ -232,6 +232,13 @@ inline int coarse_elem_occ()
     }();
     return occ;
 }
+// level 0 in one pass for nv right-hand sides in type T (the rule and its figures: packed_op)
+template <typename T>
+inline bool level0_one_wave(const top_solver *s, const DevLevel &lv, int nv)
+{
+    const dim3 one = coarse_tile_grid(lv.g);
+    return s->coarseTwoPassMin < 0 && (int64_t)one.x * one.y * (sizeof(T) == 4 ? nv : 1) <= 4 * (int64_t)s->numSMs;
+}
 // y-epilogue applied to (K in)(node) for every node of a level with packed
 // element matrices, nv right-hand sides in one launch (vectors at the
 // functors' strides): two passes, or the one-pass tile kernel (the same sums;
@@ -255,9 +262,7 @@ inline void packed_op(top_solver *s, DevLevel &lv, const In &in, const Out &out,
     int t0 = 0, nt = 0;
     coarse_elem_tiles(lv.g, t0, nt);
     T *W = wbuf<T>(lv);
-    const dim3 one = coarse_tile_grid(lv.g);
-    const int64_t oneCtas = (int64_t)one.x * one.y * (sizeof(T) == 4 ? nv : 1);
-    const bool oneWave = s->coarseTwoPassMin < 0 && &lv == &s->L[0] && oneCtas <= 4 * (int64_t)s->numSMs;
+    const bool oneWave = &lv == &s->L[0] && level0_one_wave<T>(s, lv, nv);
     if (W && s->opErr && nt > 0 && nt >= s->coarseTwoPassMin && !oneWave && coarse_elem_occ<T, In>() > 0) {
         const int64_t wvs = w_alloc_vals(lv.g.cs);
         const unsigned ctas = (unsigned)std::min<int64_t>(nt, (int64_t)s->numSMs * coarse_elem_occ<T, In>());
@@ -268,7 +273,8 @@ inline void packed_op(top_solver *s, DevLevel &lv, const In &in, const Out &out,
         launch_k(s, coarse_gather_kernel<T, Out>, dim3((unsigned)lv.g.nbx, (unsigned)lv.g.NZ, (unsigned)nv), kNodeThreads, 0, s->st,
                  out, W, wvs, lv.g, red, done);
     } else {
-        launch_k(s, coarse_tile_kernel<T, In, Out>, dim3(one.x, one.y, (unsigned)nv), dim3(kCoarseTileX, 8), 0, s->st, in, out, ks_packed<T>(lv), lv.g, red, done);
+        dim3 gr = coarse_tile_grid(lv.g); gr.z = (unsigned)nv;
+        launch_k(s, coarse_tile_kernel<T, In, Out>, gr, dim3(kCoarseTileX, 8), 0, s->st, in, out, ks_packed<T>(lv), lv.g, red, done);
     }
     TOPGPU_COUNT_LAUNCH();
 }
