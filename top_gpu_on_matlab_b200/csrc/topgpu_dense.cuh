@@ -40,6 +40,7 @@
 #include <cstdint>
 #include "topgpu_kernels.cuh"
 #include "topgpu_grid.cuh"
+#include "topgpu_streams.h"
 
 namespace topgpu {
 
@@ -633,6 +634,61 @@ inline int inverse_columns(const double *L, double *W, double *T, const double *
         }
     }
     return launches;
+}
+
+
+// The factor of A (n x n, lower part) over A and W = L^-1, on st and (n > kPb) the
+// streams of f; T: n x n scratch, Dinv: 32 x 32 values a block of 32 columns.  Each
+// step's trailing update is split: the next step's 128 columns first, on st, then the
+// rest on f.aux, beside the next diagonal block (one CTA, 37 us) and panel, which
+// touch other columns.  beside: W follows on f.inv, which reads finished columns
+// alone and writes W and T; else after the factor.  st has waited for all of it at
+// the end.  Up to kBesideMaxDofs the steps' chain leaves the chip idle and W is
+// formed beside it (assembly, n = 675 706 -> 669 us, n = 1386 1.10 -> 1.08 ms); where
+// the trailing updates fill the chip it is slower (n = 4131 5.15 ms after the factor,
+// 5.48 beside it).  Between 1386 and 4131 the line was not looked for; it lies
+// nearer the size at which the gain had shrunk to 2 %.
+constexpr int64_t kBesideMaxDofs = 2000;
+inline cudaError_t factor_and_inverse(double *A, double *W, double *T, double *Dinv, int64_t n, int *status, int sms, bool beside,
+                                      cudaStream_t st, const FactorStreams &f, int64_t &launches)
+{
+    cudaStream_t si = beside ? f.inv : st;
+    cudaError_t err = cudaSuccess;
+    auto ok = [&](cudaError_t e) { if (err == cudaSuccess) err = e; return err == cudaSuccess; };
+    auto reached = [&](cudaStream_t other) {           // other waits for what st holds so far
+        return ok(cudaEventRecord(f.go, st)) && ok(cudaStreamWaitEvent(other, f.go, 0));
+    };
+    if (beside && !reached(si)) return err;
+    if (!ok(cudaMemsetAsync(W, 0, sizeof(double) * n * n, si))) return err;
+    constexpr int kNext = kPb / kTileB;                // tile columns of the next step
+    bool restRuns = false;
+    for (int64_t k0 = 0; k0 < n; k0 += kPb) {
+        chol_diag_kernel<<<1, kDiagThreads, kDiagSmem, st>>>(A, n, k0, Dinv, status);
+        ++launches;
+        const int64_t rest = n - k0 - kPb;
+        const int nt = rest > 0 ? (int)((rest + kTileB - 1) / kTileB) : 0;
+        if (rest > 0) {
+            chol_panel(A, n, k0, Dinv, sms, st);
+            ++launches;
+        }
+        if (beside && !reached(si)) return err;
+        if (rest > 0) {
+            if (nt > kNext && !reached(f.aux)) return err;
+            if (restRuns && !ok(cudaStreamWaitEvent(st, f.auxDone, 0))) return err;      // the previous step's updates of these columns
+            chol_next(A, n, k0, st);
+            ++launches;
+            restRuns = nt > kNext;
+            if (restRuns) {
+                chol_trail_kernel<<<dim3((unsigned)nt, (unsigned)(nt - kNext)), kTileThreads, 0, f.aux>>>(A, n, k0, kNext);
+                ++launches;
+                if (!ok(cudaEventRecord(f.auxDone, f.aux))) return err;
+            }
+        }
+        if (beside) launches += inverse_columns(A, W, T, Dinv, n, k0, std::min(n, k0 + kPb), si);
+    }
+    if (!beside) launches += inverse_columns(A, W, T, Dinv, n, 0, n, st);
+    if (beside && ok(cudaEventRecord(f.invDone, si))) ok(cudaStreamWaitEvent(st, f.invDone, 0));
+    return err;
 }
 
 }  // namespace topgpu

@@ -1422,11 +1422,7 @@ extern "C" int top_solver_destroy(top_solver *s)
     if (s->capStream) cudaStreamDestroy(s->capStream);
     if (s->capIn) cudaEventDestroy(s->capIn);
     if (s->capOut) cudaEventDestroy(s->capOut);
-    if (s->auxStream) cudaStreamDestroy(s->auxStream);
-    if (s->auxGo) cudaEventDestroy(s->auxGo);
-    if (s->auxDone) cudaEventDestroy(s->auxDone);
-    if (s->invStream) cudaStreamDestroy(s->invStream);
-    if (s->invDone) cudaEventDestroy(s->invDone);
+    s->factor.destroy();
     for (auto &k : s->l0k) {
         if (k.mask) cudaFree(k.mask);
         if (k.rng) cudaFree(k.rng);
@@ -1683,60 +1679,10 @@ int coarsest_inverse(top_solver *s, cudaStream_t st)
     double *A = s->Ac;
     static const bool attr = chol_smem_attr() == cudaSuccess;
     if (!attr) { set_error("top_solver_assemble: shared memory of the coarsest factorisation"); return TOP_ERR_CUDA; }
-    // Each step's trailing update is split: the next step's 128 columns first, on
-    // the caller's stream, then the rest on a second stream, beside the next
-    // diagonal block (one CTA, 37 us) and panel, which touch other columns.  W = L^-1
-    // follows on a third stream: it reads finished columns alone and writes W and,
-    // for its products' first halves, the buffer of the inverse.  That pays where
-    // the steps' chain leaves the chip idle (assembly, n = 675 706 -> 669 us, n = 1386
-    // 1.10 -> 1.08 ms); where the trailing updates fill it, W follows the factor
-    // (n = 4131 5.15 ms, beside it 5.48).
-    const bool beside = n > kPb && !s->symPart;
-    if (n > kPb && !s->invDone) {
-        CK(cudaStreamCreateWithFlags(&s->auxStream, cudaStreamNonBlocking));
-        CK(cudaStreamCreateWithFlags(&s->invStream, cudaStreamNonBlocking));
-        CK(cudaEventCreateWithFlags(&s->auxGo, cudaEventDisableTiming));
-        CK(cudaEventCreateWithFlags(&s->auxDone, cudaEventDisableTiming));
-        CK(cudaEventCreateWithFlags(&s->invDone, cudaEventDisableTiming));
-    }
-    cudaStream_t si = beside ? s->invStream : st;
-    auto reached = [&](cudaStream_t other) {           // other waits for what st holds so far
-        cudaError_t e = cudaEventRecord(s->auxGo, st);
-        return e == cudaSuccess ? cudaStreamWaitEvent(other, s->auxGo, 0) : e;
-    };
-    if (beside) CK(reached(si));
-    CK(cudaMemsetAsync(s->Wc, 0, sizeof(double) * n * n, si));
-    constexpr int kNext = kPb / kTileB;                // tile columns of the next step
-    bool restRuns = false;
-    for (int64_t k0 = 0; k0 < n; k0 += kPb) {
-        chol_diag_kernel<<<1, kDiagThreads, kDiagSmem, st>>>(A, n, k0, s->Dc, s->zeroDone + 1);
-        TOPGPU_COUNT_LAUNCH();
-        const int64_t rest = n - k0 - kPb;
-        const int nt = rest > 0 ? (int)((rest + kTileB - 1) / kTileB) : 0;
-        if (rest > 0) {
-            chol_panel(A, n, k0, s->Dc, s->numSMs, st);
-            TOPGPU_COUNT_LAUNCH();
-        }
-        if (beside) CK(reached(si));
-        if (rest > 0) {
-            if (nt > kNext) CK(reached(s->auxStream));
-            if (restRuns) CK(cudaStreamWaitEvent(st, s->auxDone, 0));      // the previous step's updates of these columns
-            chol_next(A, n, k0, st);
-            TOPGPU_COUNT_LAUNCH();
-            restRuns = nt > kNext;
-            if (restRuns) {
-                chol_trail_kernel<<<dim3((unsigned)nt, (unsigned)(nt - kNext)), kTileThreads, 0, s->auxStream>>>(A, n, k0, kNext);
-                TOPGPU_COUNT_LAUNCH();
-                CK(cudaEventRecord(s->auxDone, s->auxStream));
-            }
-        }
-        if (beside) s->launches += inverse_columns(A, s->Wc, s->Ainv, s->Dc, n, k0, std::min(n, k0 + kPb), si);
-    }
-    if (!beside) s->launches += inverse_columns(A, s->Wc, s->Ainv, s->Dc, n, 0, n, st);
-    if (beside) {
-        CK(cudaEventRecord(s->invDone, si));
-        CK(cudaStreamWaitEvent(st, s->invDone, 0));
-    }
+    const bool beside = n > kPb && n <= kBesideMaxDofs;
+    FactorStreams &f = s->factor;
+    if (n > kPb) CK(f.create());
+    CK(factor_and_inverse(A, s->Wc, s->Ainv, s->Dc, n, s->zeroDone + 1, s->numSMs, beside, st, f, s->launches));
     // W^T W: whole, or as packed tiles over the factor, which is no longer needed.
     // The persistent coarse V-cycle (an option) reads it whole; so does build_tail,
     // which forms it for itself.

@@ -9,6 +9,7 @@
 #include <vector>
 #include <utility>
 #include "topgpu_grid.cuh"
+#include "topgpu_streams.h"
 #include "topgpu_walsh.cuh"
 #include "topgpu_tc.cuh"
 
@@ -45,8 +46,7 @@ struct top_solver {
     };
     std::vector<PcgGraph> graphs;    // one per (right-hand side, solution) pair in use
     cudaStream_t capStream = nullptr; cudaEvent_t capIn = nullptr, capOut = nullptr;
-    // the coarsest factorisation's other streams: trailing updates beside the next diagonal block, and the inverse
-    cudaStream_t auxStream = nullptr, invStream = nullptr; cudaEvent_t auxGo = nullptr, auxDone = nullptr, invDone = nullptr;
+    topgpu::FactorStreams factor;    // the coarsest factorisation's other streams
     bool useGraphs = true;
     bool coarseLanes = std::getenv("TOPGPU_COARSE_LANES") != nullptr;   // 8-lanes-per-node coarse kernel
     int coarsePersistent = 0;        // levels from 1 (1) or from 2 (2) down of the V-cycle in one cooperative launch; 0 off
