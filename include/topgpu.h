@@ -359,8 +359,9 @@ int top_solver_set_pcg_beta(top_solver *s, int flexible);
  * Takes effect at once on an assembled solver.  No counterpart in the
  * reference. */
 int top_solver_set_tail_operator(top_solver *s, int on, int *level);
-/* Test of the coarse product's failure path: the next two-pass coarse
- * product withholds one packed-tile copy, so that copy's bounded wait
+/* Test of the coarse products' failure path: the next two-pass coarse
+ * product, or packed coarsest product where none runs before it,
+ * withholds one packed-tile copy, so that copy's bounded wait
  * (one second) runs out; the kernel raises its error flag and the calling
  * entry point (top_solver_pcg, _vcycle, _matvec) returns TOP_ERR_CUDA with
  * the message set.  One-shot; the solver stays usable.  No counterpart in

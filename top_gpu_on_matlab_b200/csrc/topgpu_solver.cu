@@ -261,7 +261,9 @@ coarsest_gemv_kernel(const double *__restrict__ Ainv, const T *__restrict__ r, i
 // Each tile's two partial vectors go to part[rhs][tile][2][64]; sym_sum_kernel
 // adds a row's over the tiles in order (deterministic).  Measured (FP64 PCG,
 // iteration, whole -> packed): 4131 DOFs 216.7 -> 195.2 us, 2496 154.1 -> 141.8,
-// 1617 120.4 -> 117.2, 675 84.0 -> 86.4: from 2000 DOFs on.
+// 1617 120.4 -> 117.2, 675 84.0 -> 86.4.  The times cross near 1400 DOFs; the line
+// stands above that, where packing is worth 5 % of an iteration and more, and
+// leaves 1400 to 2000 (up to 3 %) to the one launch that reads A^-1 whole.
 constexpr int64_t kSymMinDofs = 2000;
 constexpr int kSymT = kTileB, kSymThreads = 2 * kSymT;
 constexpr uint32_t kSymTileBytes = sizeof(double) * kSymT * kSymT;
@@ -276,7 +278,7 @@ __device__ __forceinline__ void sym_tile(int t, int &I, int &J)
 template <typename T>
 __global__ void __launch_bounds__(kSymThreads)
 sym_gemv_kernel(const double *__restrict__ P, const T *__restrict__ rc, int64_t n, int tiles, double *__restrict__ part,
-                const int *__restrict__ done0, int nv, int *err)
+                const int *__restrict__ done0, int nv, int *err, int withhold)
 {
     pdl_enter();
     extern __shared__ __align__(128) unsigned char sym_smem[];
@@ -295,6 +297,7 @@ sym_gemv_kernel(const double *__restrict__ P, const T *__restrict__ rc, int64_t 
     auto issue = [&](int tile, int slot) {
         if (t != 0 || tile >= tiles) return;
         bulk::arrive_expect(bar + 8 * slot, kSymTileBytes);
+        if (withhold && tile == 0) return;   // the failure-path test: block 0's first tile never arrives
         bulk::copy(bulk::smem_addr(buf + slot * kSymT * kSymT), P + (int64_t)tile * kSymT * kSymT, kSymTileBytes, bar + 8 * slot);
     };
     for (int v0 = 0; v0 < nv; v0 += 4) {
@@ -330,7 +333,7 @@ sym_gemv_kernel(const double *__restrict__ P, const T *__restrict__ rc, int64_t 
                 if (t == 0) {
                     atomicExch(err, 1);
                     // this tile and the next may still be landing: wait for them (bounded)
-                    (void)bulk::wait(bar + 8 * (k & 1), (uint32_t)(k >> 1) & 1u);
+                    if (!(withhold && tile == 0)) (void)bulk::wait(bar + 8 * (k & 1), (uint32_t)(k >> 1) & 1u);
                     if (tile + (int)gridDim.x < tiles) (void)bulk::wait(bar + 8 * ((k + 1) & 1), (uint32_t)((k + 1) >> 1) & 1u);
                 }
                 return;
@@ -958,7 +961,8 @@ void vcycle(top_solver *s, const TR *r0, TZ *z0, double *zr, const int *done, in
         if (s->symPart) {
             const int nt = (int)((n + kSymT - 1) / kSymT), tiles = nt * (nt + 1) / 2;
             launch_k(s, sym_gemv_kernel<T>, (unsigned)std::min(tiles, 3 * s->numSMs), kSymThreads, kSymSmem, s->st,
-                     (const double *)s->Ac, rc, n, tiles, s->symPart, done, nv, s->opErr);
+                     (const double *)s->Ac, rc, n, tiles, s->symPart, done, nv, s->opErr, s->withholdTile ? 1 : 0);
+            s->withholdTile = false;
             TOPGPU_COUNT_LAUNCH();
             launch_k(s, sym_sum_kernel<T>, dim3((unsigned)nt, K), 4 * kSymT, 0, s->st,
                      (const double *)s->symPart, n, tiles, vt<T>(lc), lc.g, lc.nodeGrid, done, lvs(lc));

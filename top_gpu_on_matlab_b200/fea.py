@@ -373,8 +373,9 @@ class Solver:
         return level.value
 
     def test_withhold_tile(self):
-        """Arm the coarse product's failure-path test: the next two-pass
-        coarse product withholds one tile copy and the call reports it."""
+        """Arm the coarse products' failure-path test: the next two-pass
+        coarse product (or packed coarsest product where none runs before
+        it) withholds one tile copy and the call reports it."""
         check(lib().top_solver_test_withhold_tile(self._h), "top_solver_test_withhold_tile")
 
     def set_graphs(self, on):
