@@ -89,3 +89,32 @@ def test_pcg_with_void_chunks(name, mixed):
         # the solve's own (recurrence's) residual, converged or at the iteration
         # limit; the true one follows it to rounding
         assert float(r.norm()) < 2 * res[k] * float(b.norm())
+
+
+@pytest.mark.parametrize("mixed", [False, True])
+@pytest.mark.parametrize("name", ["slab", "corner", "two"])
+def test_same_model_in_a_larger_box(name, mixed):
+    """The model with 17 more void layers around it in z (the node order is the
+    same): equal products, V-cycles to rounding, and each solver's solution
+    solves the other's system."""
+    from top_gpu_on_matlab_b200.fea import Mesh, Solver
+    m = _mask(name)
+    sol = []
+    for extra in (0, 17):
+        mk = np.concatenate([m, np.zeros(m.shape[:2] + (extra,), bool)], 2)
+        mesh = Mesh(mk, control=400)
+        fix, ld = _bc(m, mesh, 1)
+        mesh.apply_bc(fix, ld)
+        s = Solver(mesh, E0=1.0, Emin=1e-9, penal=3.0, tol=1e-9, maxIT=800, omega=0.4, mixed=mixed)
+        s.set_density(torch.from_numpy(0.4 + 0.6 * np.random.default_rng(4).random(s.num_design)).cuda())
+        s.assemble()
+        u = torch.from_numpy(np.random.default_rng(5).standard_normal(s.numDOFs)).cuda()
+        U, _, res = s.pcg(0)
+        assert res < 1e-9
+        sol.append((s, s.matvec(0, u), s.vcycle(u), U))
+    (s0, y0, z0, U0), (s1, y1, z1, U1) = sol
+    assert torch.equal(y0, y1)
+    assert float((z0 - z1).abs().max()) < (1e-5 if mixed else 1e-11) * float(z0.abs().max())
+    b = torch.from_numpy(s0.mesh.get(0, "F")).cuda()
+    for s, U in ((s0, U1), (s1, U0)):
+        assert float((b - s.matvec(0, U)).norm()) < 2e-9 * float(b.norm())
